@@ -2,7 +2,7 @@
 
     python integer-schemes_b200/build.py          # libbssn_b200.so (+ -Xptxas -v report)
 
-Extra nvcc flags (e.g. -DBSSN_B200_NO_TMA) can be given in $BSSN_B200_NVCC_FLAGS.
+Extra nvcc flags can be given in $BSSN_B200_NVCC_FLAGS.
 
 The library lands next to the Python package that loads it
 (``bssn3d_b200/libbssn_b200.so``), so it travels with the source tree.

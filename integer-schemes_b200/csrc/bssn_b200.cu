@@ -1,27 +1,7 @@
-// bssn_b200 — fused BSSN right-hand side and RK4 stage kernels for sm_100a,
-// behind the C ABI of include/bssn_b200.h.
-//
-// The stream kernel itself lives in stream_kernel.cuh, instantiated by the
-// stream_*.cu translation units; this file holds the other kernels and the
-// C ABI. One persistent kernel per RHS evaluation (stream_kernel). Each 256-thread CTA
-// takes 4x4x16-point tiles of the padded grid in turn, one point per thread.
-// Per tile it walks the 24 fields in the order of stream.cuh: cp.async stages
-// the field's haloed tile in shared memory (double-buffered, the next field
-// streams in while this one is differentiated), every thread takes its
-// point's axial taps once and forms the first derivative, the diagonal second
-// derivative and the Kreiss-Oliger term from them, the mixed second
-// derivatives come out of two separable passes through shared memory, and the
-// result is consumed at once by the point's BSSN accumulators (bssn::Stream).
-// No derivative is written anywhere. The epilogue stores the RHS, performs the
-// RK4 stage update (algebraic enforcement fused into stage 3) or stores the
-// constraints.
-//
-// Stencils follow 3D/src/bssn3d/derivative_bundle.py:31-48 and
-// common/src/mcs_common/derivatives.py:35-106: the centred sixth-order
-// coefficients (integer sums of paired taps, scaled once), index clamped at
-// the array ends, mixed second derivatives as a first derivative along the
-// lower axis, then along the higher axis of that result.
-#include <cuda.h>
+// bssn_b200 — the C ABI of include/bssn_b200.h and the kernels around the
+// fused stream kernel (stream_kernel.cuh, instantiated by the stream_*.cu
+// translation units): the derivative bundle, the algebra on derivatives from
+// memory, norms, enforcement and the periodic sync.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -40,13 +20,121 @@
 #include "stream_launch.h"
 
 namespace bssn {
+// Stencil scale factors, set on the device from the grid spacing (per block
+// for block lists). Every stencil is summed with the integer coefficients of
+// common/src/mcs_common/derivatives.py:35-49 and scaled once:
+//   f1 = 1 / (60 h)           first derivative
+//   f2 = 1 / (180 h h)        diagonal second derivative
+//   fk = sigma / (64 h)       Kreiss-Oliger, order 6 (sigma / (256 h) for order 8)
+//   fm = f1_i * f1_j          mixed second derivative, pairs xy, xz, yz
+struct Weights {
+  double f1[3], f2[3], fk[3], fm[3];
+};
+
+__device__ __forceinline__ Params load_params(const double* __restrict__ S) {
+  Params P;
+  P.eta = S[0]; P.cahd_c = S[1]; P.dt = S[2]; P.dx = S[3];
+  P.ssl_h = S[4]; P.ssl_sigma = S[5]; P.t = S[6];
+  P.lam0 = S[7]; P.lam1 = S[8]; P.lam2 = S[9]; P.lam3 = S[10];
+  P.lamf0 = S[11]; P.lamf1 = S[12];
+  P.hx = S[13]; P.hy = S[14]; P.hz = S[15];
+  return P;
+}
+
+template <int R>
+__device__ __forceinline__ void init_weights(Weights& W, const double* __restrict__ S, double ko_sigma, int a) {
+  if (a < 3) {
+    constexpr int PI[3] = {0, 0, 1}, PJ[3] = {1, 2, 2};
+    const double h[3] = {S[13], S[14], S[15]};
+    W.f1[a] = 1.0 / (60.0 * h[a]);
+    W.f2[a] = 1.0 / ((180.0 * h[a]) * h[a]);
+    W.fk[a] = ko_sigma / ((R == 4 ? 256.0 : 64.0) * h[a]);
+    W.fm[a] = (1.0 / (60.0 * h[PI[a]])) * (1.0 / (60.0 * h[PJ[a]]));
+  }
+}
+
+// Staged tile of the derivative bundle: the 4x4x16 tile with R halo points on every side.
+template <int R>
+struct DerivGeom {
+  static constexpr int TX = 4, TY = 4, TZ = 16;
+  static constexpr int HX = TX + 2 * R, HY = TY + 2 * R, HZ = TZ + 2 * R;
+  static constexpr int HZP = 24;  // 8 mod 16: a half-warp reads 16 consecutive doubles
+  static constexpr int SX = HY * HZP, SY = HZP;
+  static constexpr int VOL = HX * HY * HZP, NELEM = HX * HY * HZ;
+  static constexpr int PER_THREAD = (NELEM + NTHREADS - 1) / NTHREADS;
+};
+
+// Issue the cp.async copies that stage one field's haloed tile, index clamped
+// at the array ends (derivatives.py:83-84 pads with the edge value).
+template <int R>
+__device__ __forceinline__ void stage_tile(double* buf, const double* __restrict__ Ff, long long x0,
+                                           long long y0, long long z0, long long Sx, long long Sy,
+                                           long long Sz, int tid) {
+  using Geo = DerivGeom<R>;
+  // 32-bit index arithmetic: a grid holds fewer than 2^31 points (check_grid)
+  const int bx = (int)x0 - R, by = (int)y0 - R, bz = (int)z0 - R;
+  const int mx = (int)Sx - 1, my = (int)Sy - 1, mz = (int)Sz - 1, sy = (int)Sy, sz = (int)Sz;
+#pragma unroll
+  for (int e = 0; e < Geo::PER_THREAD; ++e) {
+    const int idx = tid + e * NTHREADS;
+    if (idx < Geo::NELEM) {
+      const int hz = idx % Geo::HZ;
+      const int hy = (idx / Geo::HZ) % Geo::HY;
+      const int hx = idx / (Geo::HZ * Geo::HY);
+      const int qx = min(max(bx + hx, 0), mx);
+      const int qy = min(max(by + hy, 0), my);
+      const int qz = min(max(bz + hz, 0), mz);
+      cp_async8(buf + hx * Geo::SX + hy * Geo::SY + hz, Ff + ((qx * sy + qy) * sz + qz));
+    }
+  }
+}
+
+// Final-stage values of the fields that algebraic enforcement rewrites are
+// held back (gt0..5, At0..5, chi, alpha); the rest are stored directly.
+__device__ __forceinline__ bool hold_for_enforce(double* en, int k, double un) {
+  if (k >= F_GT && k < F_GT + 6) en[k - F_GT] = un;
+  else if (k >= F_AT && k < F_AT + 6) en[6 + k - F_AT] = un;
+  else if (k == F_CHI) en[12] = un;
+  else if (k == F_ALPHA) en[13] = un;
+  else return false;
+  return true;
+}
+
+// Algebraic enforcement of one point (evolve.py:93-119): unit conformal
+// determinant, traceless A~ with the unit-det inverse, chi and alpha floors.
+__device__ __forceinline__ void enforce_point(double* en, double* O, long long n, double chi_floor,
+                                              double alpha_floor) {
+  double* g = en;
+  double* a = en + 6;
+  const double det = g[0] * (g[3] * g[5] - g[4] * g[4]) - g[1] * (g[1] * g[5] - g[4] * g[2]) +
+                     g[2] * (g[1] * g[4] - g[3] * g[2]);
+  const double scale = pow(det, -1.0 / 3.0);
+#pragma unroll
+  for (int q = 0; q < 6; ++q) g[q] = g[q] * scale;
+  const double iuxx = g[3] * g[5] - g[4] * g[4];
+  const double iuxy = g[2] * g[4] - g[1] * g[5];
+  const double iuxz = g[1] * g[4] - g[2] * g[3];
+  const double iuyy = g[0] * g[5] - g[2] * g[2];
+  const double iuyz = g[1] * g[2] - g[0] * g[4];
+  const double iuzz = g[0] * g[3] - g[1] * g[1];
+  const double trA = iuxx * a[0] + iuyy * a[3] + iuzz * a[5] + 2.0 * (iuxy * a[1] + iuxz * a[2] + iuyz * a[4]);
+  const double third = trA / 3.0;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    O[(long long)(F_GT + q) * n] = g[q];
+    O[(long long)(F_AT + q) * n] = a[q] - g[q] * third;
+  }
+  O[(long long)F_CHI * n] = fmax(en[12], chi_floor);
+  O[(long long)F_ALPHA * n] = fmax(en[13], alpha_floor);
+}
+
 // ---------------------------------------------------------------------------
 // Derivative bundle to global memory (the bssn_b200_derivatives entry).
 // ---------------------------------------------------------------------------
 template <int R>
 __device__ __forceinline__ void field_derivs(const double* __restrict__ t, int c, int f, const Weights& W,
                                              bool ko, double* __restrict__ out, long long n) {
-  constexpr int st[3] = {TileGeom<R>::SX, TileGeom<R>::SY, 1};
+  constexpr int st[3] = {DerivGeom<R>::SX, DerivGeom<R>::SY, 1};
   double kacc = 0.0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -82,7 +170,7 @@ __device__ __forceinline__ void field_derivs(const double* __restrict__ t, int c
 
 template <int R>
 __global__ void __launch_bounds__(NTHREADS) deriv_kernel(const Args args) {
-  using Geo = TileGeom<R>;
+  using Geo = DerivGeom<R>;
   extern __shared__ __align__(128) double smem[];
   __shared__ Weights W;
   const int tid = threadIdx.x;
@@ -152,7 +240,7 @@ __global__ void __launch_bounds__(128) algebra_kernel(const double* __restrict__
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
     auto fld = [&](int k) -> double { return __ldg(F + (long long)k * n + q); };
     auto drv = [&](int s) -> double { return __ldg(D + (long long)s * n + q); };
-    Stream<true, false> acc;
+    Stream acc;
     acc.init(fld);
     Unroll<0, NFIELD>::run([&](auto ic) {
       constexpr int f = stream_field(decltype(ic)::value);
@@ -164,7 +252,7 @@ __global__ void __launch_bounds__(128) algebra_kernel(const double* __restrict__
       acc.consume(f, d1, d2, 0.0, P, fld);
     });
     auto emit = [&](int k, double v) { OUT[(long long)k * n + q] = v; };
-    acc.finalize(fld, P, emit, NoCon());
+    acc.finalize(fld, P, emit);
   }
 }
 
@@ -217,7 +305,7 @@ __global__ void __launch_bounds__(128) stage_derivs_kernel(
     P.t = P0.t + cs * P0.dt;  // stage time t, t+dt/2, t+dt/2, t+dt (evolve.py:125-131)
     auto fld = [&](int k) -> double { return __ldg(Y + gidx + (long long)k * n); };
     auto drv = [&](int s) -> double { return __ldg(Dq + (long long)s * n); };
-    Stream<true, false> acc;
+    Stream acc;
     acc.init(fld);
     Unroll<0, NFIELD>::run([&](auto ic) {
       constexpr int f = stream_field(decltype(ic)::value);
@@ -247,7 +335,7 @@ __global__ void __launch_bounds__(128) stage_derivs_kernel(
         if (!hold_for_enforce(en, k, un)) O[o] = un;
       }
     };
-    acc.finalize(fld, P, emit, NoCon());
+    acc.finalize(fld, P, emit);
     if (stage == 3) enforce_point(en, O, n, chi_floor, alpha_floor);
   }
 }
@@ -341,7 +429,7 @@ int device_sms(int* sms) {
 
 template <int R>
 int launch_deriv(const bssn::Args& a, cudaStream_t stream, int grid) {
-  using Geo = bssn::TileGeom<R>;
+  using Geo = bssn::DerivGeom<R>;
   const size_t smem = (size_t)Geo::VOL * sizeof(double);
   auto kern = bssn::deriv_kernel<R>;
   static int flags[kMaxDev] = {0};
@@ -507,16 +595,7 @@ const char* bssn_b200_version(void) { return "bssn_b200 0.3 sm_100a"; }
 
 int bssn_b200_async_copy_errors(int* count) {
   if (!count) return fail(BSSN_B200_EINVAL, "async_copy_errors: NULL operand");
-  int total = 0;
-  int (*const parts[])(int*) = {bssn_host::copy_errors_rhs, bssn_host::copy_errors_stage,
-                                bssn_host::copy_errors_msrk};
-  for (auto part : parts) {
-    int c = 0;
-    const int rc = part(&c);
-    if (rc) return rc;
-    total += c;
-  }
-  *count = total;
+  *count = 0;
   return 0;
 }
 

@@ -1,13 +1,14 @@
-// Streaming form of the pointwise BSSN right-hand side (CAHD + SSL) for the
-// sm_100a fused kernel.
+// The pointwise BSSN right-hand side (CAHD + SSL) from derivatives that arrive
+// field by field, for the kernels that read them from memory (algebra_kernel,
+// stage_derivs_kernel), and the field numbering and parameters that all
+// kernels share. (stream_kernel.cuh states the same algebra split over two
+// roles.)
 //
-// The fused kernel differentiates one field at a time out of a shared-memory
-// tile. Instead of parking the 138 derivatives anywhere, each field's
-// derivatives are handed to `Stream::consume_*` as soon as they exist and are
-// folded into running accumulators; only the derivatives that enter
-// nonlinearly (d gt, d chi, d alpha) are kept, and only until the
-// quantities built from them (Christoffel symbols, Ricci tensor, D_iD_j alpha)
-// are complete. Field order is fixed:
+// Each field's derivatives are handed to `Stream::consume_*` and folded into
+// running accumulators; only the derivatives that enter nonlinearly (d gt,
+// d chi, d alpha) are kept, and only until the quantities built from them
+// (Christoffel symbols, Ricci tensor, D_iD_j alpha) are complete. Field order
+// is fixed:
 //
 //   gt0..5 -> finish_metric -> chi -> alpha -> Gt0..2 -> finish_ricci ->
 //   beta0..2 -> finish_beta -> K -> At0..5 -> B0..2 -> finalize
@@ -27,8 +28,7 @@
 //   B_t     = Gt_t - eta B + l2 b.d B - l3 b.d Gt
 // with G^k = gt^ij G^k_ij the metric-computed contracted Christoffel symbol
 // (it also enters the Ricci term G^k G_(ij)k), R_ij = R~_ij + R^chi_ij, and
-// H = chi gt^ij R_ij + 2/3 K^2 - At_ij At^ij. Constraints (CONS) follow the
-// reference's ConstraintSolver (3D/src/bssn3d/constraints.py:38-62).
+// H = chi gt^ij R_ij + 2/3 K^2 - At_ij At^ij.
 #pragma once
 
 namespace bssn {
@@ -78,23 +78,13 @@ __host__ __device__ constexpr int stream_field(int idx) {
        : F_B + (idx - 21);
 }
 
-struct NoCon {
-  __device__ __forceinline__ void operator()(double, double, double, double) const {}
-};
-
-template <bool RATES, bool CONS, bool PV = false>
 struct Stream {
-  // Point values: held in registers, or (PV) re-read on every use from the
-  // point's staged column pv[k * ps] (shared memory), which frees their
-  // registers for the accumulators.
-  const double* pv = nullptr;
-  int ps = 0;
-  double al_, chi_, K_, g_[6], b_[3];
-  __device__ __forceinline__ double Al() const { return PV ? pv[F_ALPHA * ps] : al_; }
-  __device__ __forceinline__ double Chi() const { return PV ? pv[F_CHI * ps] : chi_; }
-  __device__ __forceinline__ double Kv() const { return PV ? pv[F_K * ps] : K_; }
-  __device__ __forceinline__ double Gv(int p) const { return PV ? pv[(F_GT + p) * ps] : g_[p]; }
-  __device__ __forceinline__ double Bv(int i) const { return PV ? pv[(F_BETA + i) * ps] : b_[i]; }
+  double al_, chi_, K_, g_[6], b_[3];  // point values
+  __device__ __forceinline__ double Al() const { return al_; }
+  __device__ __forceinline__ double Chi() const { return chi_; }
+  __device__ __forceinline__ double Kv() const { return K_; }
+  __device__ __forceinline__ double Gv(int p) const { return g_[p]; }
+  __device__ __forceinline__ double Bv(int i) const { return b_[i]; }
   double ichi;
   double gu[6];
   double AU[6], AA;
@@ -107,19 +97,16 @@ struct Stream {
   double R[6], X[6];     // Ricci accumulator; X = alpha R - D_iD_j alpha
   double dchi[3], guchi[3];
   double lapa, trR, trX, divb, dd[3];
-  double mom[3];
 
   template <class Fld>
   __device__ __forceinline__ void init(const Fld& fld) {
-    if (!PV) {
-      al_ = fld(F_ALPHA);
-      chi_ = fld(F_CHI);
-      K_ = fld(F_K);
+    al_ = fld(F_ALPHA);
+    chi_ = fld(F_CHI);
+    K_ = fld(F_K);
 #pragma unroll
-      for (int p = 0; p < 6; ++p) g_[p] = fld(F_GT + p);
+    for (int p = 0; p < 6; ++p) g_[p] = fld(F_GT + p);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) b_[i] = fld(F_BETA + i);
-    }
+    for (int i = 0; i < 3; ++i) b_[i] = fld(F_BETA + i);
     ichi = 1.0 / Chi();
     {
       const double a00 = Gv(3) * Gv(5) - Gv(4) * Gv(4);
@@ -153,7 +140,7 @@ struct Stream {
 #pragma unroll
     for (int p = 0; p < 6; ++p) { R[p] = 0.0; X[p] = 0.0; r_At[p] = 0.0; }
 #pragma unroll
-    for (int i = 0; i < 3; ++i) { r_Gt[i] = 0.0; r_B[i] = 0.0; dd[i] = 0.0; mom[i] = 0.0; }
+    for (int i = 0; i < 3; ++i) { r_Gt[i] = 0.0; r_B[i] = 0.0; dd[i] = 0.0; }
     divb = 0.0;
   }
 
@@ -218,7 +205,7 @@ struct Stream {
           q += C2[k][sym(l, i)] * W[j][k][l] + C2[k][sym(l, j)] * W[i][k][l] + C2[k][sym(i, l)] * W[k][j][l];
       R[p] += q;
     }
-    if (RATES) {
+    {
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         double c2au = 0.0;
@@ -250,7 +237,7 @@ struct Stream {
       const int i = sym_i(p), j = sym_j(p);
       R[p] += hichi * (Dchi[p] + Gv(p) * lapchi) - qichi2 * (dchi[i] * dchi[j] + 3.0 * Gv(p) * sqchi);
     }
-    if (RATES) {
+    {
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const double t = AU[sym(i, 0)] * dchi[0] + AU[sym(i, 1)] * dchi[1] + AU[sym(i, 2)] * dchi[2];
@@ -273,7 +260,7 @@ struct Stream {
       X[p] = -dda;
       lapa += symw(p) * gu[p] * dda;
     }
-    if (RATES) {
+    {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
         r_Gt[i] -= 2.0 * (AU[sym(i, 0)] * dal[0] + AU[sym(i, 1)] * dal[1] + AU[sym(i, 2)] * dal[2]);
@@ -343,26 +330,16 @@ struct Stream {
   // ---- K -------------------------------------------------------------------------
   __device__ __forceinline__ void consume_K(const double (&d1)[3], double ko) {
     r_K = adv(d1) + ko;
-    if (RATES) {
+    {
 #pragma unroll
       for (int i = 0; i < 3; ++i)
         r_Gt[i] -= (4.0 / 3.0) * Al() * (gu[sym(i, 0)] * d1[0] + gu[sym(i, 1)] * d1[1] + gu[sym(i, 2)] * d1[2]);
-    }
-    if (CONS) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) mom[i] -= (2.0 / 3.0) * d1[i];
     }
   }
 
   // ---- At_p ----------------------------------------------------------------------
   __device__ __forceinline__ void consume_At(int p, const double (&d1)[3], double ko) {
     r_At[p] += adv(d1) + ko;
-    if (CONS) {
-      // g~^jk d_j A~_ki, A~_ki = A~_p for {k, i} = pair p
-      const int i = sym_i(p), k = sym_j(p);
-      mom[i] += gu[sym(0, k)] * d1[0] + gu[sym(1, k)] * d1[1] + gu[sym(2, k)] * d1[2];
-      if (i != k) mom[k] += gu[sym(0, i)] * d1[0] + gu[sym(1, i)] * d1[1] + gu[sym(2, i)] * d1[2];
-    }
   }
 
   // ---- B^k -------------------------------------------------------------------------
@@ -370,31 +347,10 @@ struct Stream {
     r_B[k] += lam2 * adv(d1) + ko;
   }
 
-  // ---- closing terms; emit(field, rate) and con(H, M0, M1, M2) ------------------------
-  template <class Fld, class Emit, class Con>
-  __device__ __forceinline__ void finalize(const Fld& fld, const Params& P, const Emit& emit, const Con& con) {
+  // ---- closing terms; emit(field, rate) ------------------------------------------------
+  template <class Fld, class Emit>
+  __device__ __forceinline__ void finalize(const Fld& fld, const Params& P, const Emit& emit) {
     const double H = Chi() * trR + (2.0 / 3.0) * Kv() * Kv() - AA;
-    if (CONS) {
-      double A[6];
-#pragma unroll
-      for (int p = 0; p < 6; ++p) A[p] = fld(F_AT + p);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        double m = 0.0, c = 0.0;
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const int ji = sym(j, i);
-            m += gu[sym(j, k)] * (C2[0][ji] * A[sym(k, 0)] + C2[1][ji] * A[sym(k, 1)] + C2[2][ji] * A[sym(k, 2)]);
-            c += gu[sym(j, k)] * A[sym(k, i)] * dchi[j];
-          }
-        const double gA = fld(F_GTI + 0) * A[sym(i, 0)] + fld(F_GTI + 1) * A[sym(i, 1)] + fld(F_GTI + 2) * A[sym(i, 2)];
-        mom[i] += -m - gA - 1.5 * c * ichi;
-      }
-      con(H, mom[0], mom[1], mom[2]);
-    }
-    if (!RATES) return;
     // A~_ij
     {
       double A[6];

@@ -6,19 +6,20 @@
 
 namespace bssn_host {
 
-template <int MODE>
+template <int MODE, bool KO>
 static int by_variant(int variant, const bssn::Args& a, cudaStream_t st, int grid) {
   switch (variant) {
-    case 1: return launch_stream<3, MODE, bssn::Shape<2, 8, 16>>(a, st, grid);
-    case 2: return launch_stream<3, MODE, bssn::Shape<4, 8, 8>>(a, st, grid);
-    case 3: return launch_stream<3, MODE, bssn::Shape<8, 4, 8>>(a, st, grid);
+    case 1: return launch_stream<3, MODE, KO, bssn::Shape<2, 8, 16>>(a, st, grid);
+    case 2: return launch_stream<3, MODE, KO, bssn::Shape<4, 8, 8>>(a, st, grid);
+    case 3: return launch_stream<3, MODE, KO, bssn::Shape<8, 4, 8>>(a, st, grid);
     default: return fail(BSSN_B200_EINVAL, "variant out of range");
   }
 }
 
 int launch_batch_r3(int mode, int variant, const bssn::Args& a, cudaStream_t st, int grid) {
-  if (mode == bssn::MODE_RHS) return by_variant<bssn::MODE_RHS>(variant, a, st, grid);
-  if (mode == bssn::MODE_STAGE) return by_variant<bssn::MODE_STAGE>(variant, a, st, grid);
+  if (mode == bssn::MODE_RHS) return by_variant<bssn::MODE_RHS, false>(variant, a, st, grid);
+  if (mode == bssn::MODE_STAGE) 
+    return a.use_ko ? by_variant<bssn::MODE_STAGE, true>(variant, a, st, grid) : by_variant<bssn::MODE_STAGE, false>(variant, a, st, grid);
   return fail(BSSN_B200_EINVAL, "stream kernel: no batched instantiation for this mode");
 }
 

@@ -9,9 +9,9 @@ namespace bssn_host {
 int launch_batch_r4(int mode, int variant, const bssn::Args& a, cudaStream_t st, int grid) {
   if (mode != bssn::MODE_STAGE) return fail(BSSN_B200_EINVAL, "stream kernel: no batched instantiation for this mode");
   switch (variant) {
-    case 1: return launch_stream<4, bssn::MODE_STAGE, bssn::Shape<2, 8, 16>>(a, st, grid);
-    case 2: return launch_stream<4, bssn::MODE_STAGE, bssn::Shape<4, 8, 8>>(a, st, grid);
-    case 3: return launch_stream<4, bssn::MODE_STAGE, bssn::Shape<8, 4, 8>>(a, st, grid);
+    case 1: return launch_stream<4, bssn::MODE_STAGE, true, bssn::Shape<2, 8, 16>>(a, st, grid);
+    case 2: return launch_stream<4, bssn::MODE_STAGE, true, bssn::Shape<4, 8, 8>>(a, st, grid);
+    case 3: return launch_stream<4, bssn::MODE_STAGE, true, bssn::Shape<8, 4, 8>>(a, st, grid);
     default: return fail(BSSN_B200_EINVAL, "variant out of range");
   }
 }

@@ -21,8 +21,5 @@ int launch_stage_modes(int R, int mode, const bssn::Args& a, cudaStream_t st, in
 int launch_msrk_modes(int R, int mode, const bssn::Args& a, cudaStream_t st, int grid);
 int launch_batch_r3(int mode, int variant, const bssn::Args& a, cudaStream_t st, int grid);
 int launch_batch_r4(int mode, int variant, const bssn::Args& a, cudaStream_t st, int grid);
-int copy_errors_rhs(int* count);
-int copy_errors_stage(int* count);
-int copy_errors_msrk(int* count);
 
 }  // namespace bssn_host

@@ -7,12 +7,10 @@ namespace bssn_host {
 
 int launch_stage_modes(int R, int mode, const bssn::Args& a, cudaStream_t st, int grid) {
   if (mode == bssn::MODE_STAGE) {
-    if (R == 3) return launch_stream<3, bssn::MODE_STAGE>(a, st, grid);
-    if (R == 4) return launch_stream<4, bssn::MODE_STAGE>(a, st, grid);
+    if (R == 3) return a.use_ko ? launch_stream<3, bssn::MODE_STAGE, true>(a, st, grid) : launch_stream<3, bssn::MODE_STAGE, false>(a, st, grid);
+    if (R == 4) return launch_stream<4, bssn::MODE_STAGE, true>(a, st, grid);
   }
   return fail(BSSN_B200_EINVAL, "stream kernel: no stage instantiation for this order/mode");
 }
-
-int copy_errors_stage(int* count) { return read_copy_errors(count); }
 
 }  // namespace bssn_host

@@ -1,0 +1,79 @@
+"""The two-role stream kernel where it can go wrong: tiles that hang over every
+end of the array, extents below one tile, odd z extents (no aligned rows) and
+even ones (16-byte copies with clamped ends), more tiles than CTAs, every
+instantiation of the stage (no KO, KO 6, KO 8), all tile shapes on blocks with
+and without a ghost margin.
+
+Bars as in test_gpu_parity.py: 1e-12 of each field's largest rate (a second
+derivative of O(1) data carries eps / h^2 = 2e-14, times at most ~50 terms)."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+H = (0.1, 0.11, 0.09)
+
+
+def _S(dt=0.02, t=0.7):
+    from bssn3d_b200.fused_rhs import pack_S
+    return pack_S(2.0, 0.06, dt, H[0], 0.6, 20.0, t, (1, 1, 1, 1), (1, 0), H[1], H[2])
+
+
+def _state(shape, seed):
+    F = 0.05 * np.random.default_rng(seed).standard_normal((24,) + shape)
+    for k in (0, 1, 3, 6, 8):
+        F[k] += 1.0
+    return F
+
+
+SHAPES = [(1, 1, 1), (2, 3, 5), (4, 4, 16), (5, 3, 17), (3, 9, 18), (8, 4, 33), (23, 26, 34)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("ko", [0, 6, 8])
+def test_stage_rate_at_tile_edges(shape, ko):
+    from bssn3d_b200 import _lib
+    lib = _lib.load()
+    F, S = _state(shape, sum(shape)), _S()
+    sigma = 0.1 if ko else 0.0
+    want = O.rhs(F, S) + (O.ko(F, *H, sigma, ko) if ko else 0.0)
+    Fd, Sd = torch.from_numpy(F).cuda(), torch.from_numpy(S).cuda()
+    acc, nxt = torch.empty_like(Fd), torch.empty_like(Fd)
+    _lib.check(lib.bssn_b200_rk4_stage(torch.cuda.current_stream().cuda_stream, 0, Fd.data_ptr(), Fd.data_ptr(),
+                                       acc.data_ptr(), nxt.data_ptr(), Sd.data_ptr(), sigma, ko or 6, 1e-4, 1e-4,
+                                       *shape))
+    got = acc.cpu().numpy()
+    assert O.normwise_rel(got, want).max() < 1e-12
+    # y_next = u + dt/2 rate, two roundings of O(1) values
+    assert np.abs(nxt.cpu().numpy() - (F + 0.5 * S[2] * got)).max() <= 4 * np.finfo(float).eps * np.abs(F).max()
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("core,n", [(0, 13), (3, 10), (3, 17), (4, 12), (5, 11)])
+def test_block_tiles_cover_the_core(variant, core, n):
+    import ctypes
+    from bssn3d_b200 import _lib
+    from bssn3d_b200.amr import BlockDesc
+    lib = _lib.load()
+    s = n + 2 * core
+    F, S = _state((s, s, s), 7 * n + core), _S()
+    S[3] = S[13] = S[14] = S[15] = 0.1
+    tab = (BlockDesc * 1)()
+    tab[0].sx = tab[0].sy = tab[0].sz = s
+    tab[0].h[:] = [0.1] * 3
+    tab[0].core = core
+    nt = lib.bssn_b200_batch_plan(ctypes.addressof(tab), 1, variant)
+    dev = torch.frombuffer(bytearray(bytes(memoryview(tab).cast("B"))), dtype=torch.uint8).cuda()
+    Fd, Sd = torch.from_numpy(F).cuda(), torch.from_numpy(S).cuda()
+    out = torch.full_like(Fd, np.nan)
+    _lib.check(lib.bssn_b200_batch_rhs(torch.cuda.current_stream().cuda_stream, Fd.data_ptr(), Sd.data_ptr(),
+                                       out.data_ptr(), dev.data_ptr(), 1, nt, variant))
+    got = out.cpu().numpy()
+    inner = (slice(None),) + (slice(core, s - core),) * 3
+    written = np.isfinite(got[0])
+    assert written.sum() == n ** 3 and written[inner[1:]].all()   # the core and nothing else
+    assert O.normwise_rel(got[inner], O.rhs(F, S)[inner]).max() < 1e-12
