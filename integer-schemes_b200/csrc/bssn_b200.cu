@@ -20,17 +20,6 @@
 #include "stream_launch.h"
 
 namespace bssn {
-// Stencil scale factors, set on the device from the grid spacing (per block
-// for block lists). Every stencil is summed with the integer coefficients of
-// common/src/mcs_common/derivatives.py:35-49 and scaled once:
-//   f1 = 1 / (60 h)           first derivative
-//   f2 = 1 / (180 h h)        diagonal second derivative
-//   fk = sigma / (64 h)       Kreiss-Oliger, order 6 (sigma / (256 h) for order 8)
-//   fm = f1_i * f1_j          mixed second derivative, pairs xy, xz, yz
-struct Weights {
-  double f1[3], f2[3], fk[3], fm[3];
-};
-
 __device__ __forceinline__ Params load_params(const double* __restrict__ S) {
   Params P;
   P.eta = S[0]; P.cahd_c = S[1]; P.dt = S[2]; P.dx = S[3];
@@ -39,54 +28,6 @@ __device__ __forceinline__ Params load_params(const double* __restrict__ S) {
   P.lamf0 = S[11]; P.lamf1 = S[12];
   P.hx = S[13]; P.hy = S[14]; P.hz = S[15];
   return P;
-}
-
-template <int R>
-__device__ __forceinline__ void init_weights(Weights& W, const double* __restrict__ S, double ko_sigma, int a) {
-  if (a < 3) {
-    constexpr int PI[3] = {0, 0, 1}, PJ[3] = {1, 2, 2};
-    const double h[3] = {S[13], S[14], S[15]};
-    W.f1[a] = 1.0 / (60.0 * h[a]);
-    W.f2[a] = 1.0 / ((180.0 * h[a]) * h[a]);
-    W.fk[a] = ko_sigma / ((R == 4 ? 256.0 : 64.0) * h[a]);
-    W.fm[a] = (1.0 / (60.0 * h[PI[a]])) * (1.0 / (60.0 * h[PJ[a]]));
-  }
-}
-
-// Staged tile of the derivative bundle: the 4x4x16 tile with R halo points on every side.
-template <int R>
-struct DerivGeom {
-  static constexpr int TX = 4, TY = 4, TZ = 16;
-  static constexpr int HX = TX + 2 * R, HY = TY + 2 * R, HZ = TZ + 2 * R;
-  static constexpr int HZP = 24;  // 8 mod 16: a half-warp reads 16 consecutive doubles
-  static constexpr int SX = HY * HZP, SY = HZP;
-  static constexpr int VOL = HX * HY * HZP, NELEM = HX * HY * HZ;
-  static constexpr int PER_THREAD = (NELEM + NTHREADS - 1) / NTHREADS;
-};
-
-// Issue the cp.async copies that stage one field's haloed tile, index clamped
-// at the array ends (derivatives.py:83-84 pads with the edge value).
-template <int R>
-__device__ __forceinline__ void stage_tile(double* buf, const double* __restrict__ Ff, long long x0,
-                                           long long y0, long long z0, long long Sx, long long Sy,
-                                           long long Sz, int tid) {
-  using Geo = DerivGeom<R>;
-  // 32-bit index arithmetic: a grid holds fewer than 2^31 points (check_grid)
-  const int bx = (int)x0 - R, by = (int)y0 - R, bz = (int)z0 - R;
-  const int mx = (int)Sx - 1, my = (int)Sy - 1, mz = (int)Sz - 1, sy = (int)Sy, sz = (int)Sz;
-#pragma unroll
-  for (int e = 0; e < Geo::PER_THREAD; ++e) {
-    const int idx = tid + e * NTHREADS;
-    if (idx < Geo::NELEM) {
-      const int hz = idx % Geo::HZ;
-      const int hy = (idx / Geo::HZ) % Geo::HY;
-      const int hx = idx / (Geo::HZ * Geo::HY);
-      const int qx = min(max(bx + hx, 0), mx);
-      const int qy = min(max(by + hy, 0), my);
-      const int qz = min(max(bz + hz, 0), mz);
-      cp_async8(buf + hx * Geo::SX + hy * Geo::SY + hz, Ff + ((qx * sy + qy) * sz + qz));
-    }
-  }
 }
 
 // Final-stage values of the fields that algebraic enforcement rewrites are
@@ -129,72 +70,88 @@ __device__ __forceinline__ void enforce_point(double* en, double* O, long long n
 }
 
 // ---------------------------------------------------------------------------
-// Derivative bundle to global memory (the bssn_b200_derivatives entry).
+// Derivative bundle to global memory (the bssn_b200_derivatives entry): the
+// staging and the stencils of the stream kernel, one field at a time,
+// double-buffered, every result stored at once. 1.5 KB are written and 0.2 KB
+// read per point, so the stores should be all that counts: three CTAs per SM
+// (85 registers, 49 KB each) keep them going while others differentiate. An
+// 86^3 array with KO6: 0.64 ms with single buffering, one 8-byte copy a cell
+// and 36 taps per mixed derivative, 0.43 ms now (2.2 TB/s; copy
+// latency and the shared-memory pipe bound it).
 // ---------------------------------------------------------------------------
 template <int R>
-__device__ __forceinline__ void field_derivs(const double* __restrict__ t, int c, int f, const Weights& W,
-                                             bool ko, double* __restrict__ out, long long n) {
-  constexpr int st[3] = {DerivGeom<R>::SX, DerivGeom<R>::SY, 1};
-  double kacc = 0.0;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    double v[2 * R + 1];
-#pragma unroll
-    for (int k = 0; k <= 2 * R; ++k) v[k] = t[c + (k - R) * st[a]];
-    out[(long long)d1slot(f, a) * n] =
-        __dmul_rn(c1_sum(v[R - 3], v[R - 2], v[R - 1], v[R + 1], v[R + 2], v[R + 3]), W.f1[a]);
-    const double s1 = __dadd_rn(v[R + 1], v[R - 1]), s2 = __dadd_rn(v[R + 2], v[R - 2]),
-                 s3 = __dadd_rn(v[R + 3], v[R - 3]);
-    if (has_d2(f)) out[(long long)d2slot(f, sym(a, a)) * n] = __dmul_rn(c2_sum(v[R], s1, s2, s3), W.f2[a]);
-    if (ko) {
-      const double sk = R == 4 ? ko8_sum(v[R], s1, s2, s3, __dadd_rn(v[2 * R], v[0])) : ko6_sum(v[R], s1, s2, s3);
-      kacc = __dadd_rn(kacc, __dmul_rn(sk, W.fk[a]));
-    }
-  }
-  if (has_d2(f)) {
-    // mixed: the unscaled first-derivative sums along i at the 6 offsets along
-    // j, differentiated along j, scaled by f1_i * f1_j
-    constexpr int PI[3] = {0, 0, 1}, PJ[3] = {1, 2, 2};
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const int i = PI[q], j = PJ[q];
-      double inner[7];
-#pragma unroll
-      for (int b = 0; b < 7; ++b) inner[b] = b == 3 ? 0.0 : c1_at(t + c + (b - 3) * st[j], st[i]);
-      out[(long long)d2slot(f, sym(i, j)) * n] =
-          __dmul_rn(c1_sum(inner[0], inner[1], inner[2], inner[4], inner[5], inner[6]), W.fm[q]);
-    }
-  }
-  if (ko) out[(long long)(NDERIV + f) * n] = kacc;
-}
+struct DerivLayout {
+  using G = TileGeom<R, DefaultShape>;
+  static constexpr size_t SMEM = (size_t)(2 * G::VOL + G::TVOL) * sizeof(double) + (size_t)2 * G::NROW * sizeof(int);
+};
 
-template <int R>
-__global__ void __launch_bounds__(NTHREADS) deriv_kernel(const Args args) {
-  using Geo = DerivGeom<R>;
+template <int R, bool KO>
+__global__ void __launch_bounds__(NTHREADS, 3) deriv_kernel(const __grid_constant__ Args args) {
+  using T = DefaultShape;
+  using G = TileGeom<R, T>;
   extern __shared__ __align__(128) double smem[];
-  __shared__ Weights W;
+  __shared__ TileDesc s_desc[2];
+  double* const T1 = smem + 2 * G::VOL;
+  int* const rows = reinterpret_cast<int*>(T1 + G::TVOL);
+  double* cur = smem;
+  double* nxt = smem + G::VOL;
   const int tid = threadIdx.x;
-  init_weights<R>(W, args.S, args.ko_sigma, tid);
-  __syncthreads();
-  const long long Sx = args.Sx, Sy = args.Sy, Sz = args.Sz, n = args.n;
-  constexpr int TX = Geo::TX, TY = Geo::TY, TZ = Geo::TZ;
-  const int lz = tid % TZ, ly = (tid / TZ) % TY, lx = tid / (TZ * TY);
-  const int c = (lx + R) * Geo::SX + (ly + R) * Geo::SY + (lz + R);
+  const int lz = tid % T::Z, ly = (tid / T::Z) % T::Y, lx = tid / (T::Z * T::Y);
+  const PointPlace place = point_place<R, T>(tid);
+  const StagePlace splace = stage_place<R, T>(tid);
+  const long long n = args.n;
   const int ntiles = args.ntx * args.nty * args.ntz;
+  auto issue = [&](int f, const TileDesc& d, const int* rw, double* buf) {
+    const int z = d.zs + splace.ch;
+    if (splace.row0 < G::NROW && z < d.sz + R) {
+      const bool whole = d.al && z >= 0 && z + 1 < d.sz;
+      if (has_d2(f)) stage_rows<R, T, true>(buf, args.F + (f * n + z), rw, splace, whole, d);
+      else stage_rows<R, T, false>(buf, args.F + (f * n + z), rw, splace, whole, d);
+    }
+    cp_async_commit();
+  };
+  if (tid < 32) fill_desc<R, T>(args, blockIdx.x, &s_desc[0], nullptr);
+  __syncthreads();
+  fill_rows<R, T>(s_desc[0], rows, tid);
+  __syncthreads();
+  issue(0, s_desc[0], rows, cur);
+  int par = 0;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int tz = tile % args.ntz, ty = (tile / args.ntz) % args.nty, tx = tile / (args.ntz * args.nty);
-    const long long x0 = (long long)tx * TX, y0 = (long long)ty * TY, z0 = (long long)tz * TZ;
-    const long long gx = x0 + lx, gy = y0 + ly, gz = z0 + lz;
-    const bool inside = gx < Sx && gy < Sy && gz < Sz;
-    double* out = args.OUT + (gx * Sy + gy) * Sz + gz;
+    const TileDesc& d = s_desc[par];
+    const bool has_next = tile + (int)gridDim.x < ntiles;
+    const int gx = d.x0 + lx, gy = d.y0 + ly, gz = d.z0 + lz, dz = d.z0 - d.zs;
+    const bool inside = gx < d.sx && gy < d.sy && gz < d.sz;
+    double* const out = args.OUT + ((long long)gx * d.sy + gy) * d.sz + gz;
+#pragma unroll 1
     for (int f = 0; f < NFIELD; ++f) {
-      stage_tile<R>(smem, args.F + (long long)f * n, x0, y0, z0, Sx, Sy, Sz, tid);
-      cp_async_commit();
       cp_async_wait<0>();
       __syncthreads();
-      if (inside) field_derivs<R>(smem, c, f, W, args.use_ko != 0, out, n);
-      __syncthreads();
+      if (f + 1 < NFIELD) issue(f + 1, d, rows + par * G::NROW, nxt);
+      else if (has_next) issue(0, s_desc[par ^ 1], rows + (par ^ 1) * G::NROW, nxt);
+      if (has_next) {
+        if (f == 0 && tid < 32) fill_desc<R, T>(args, tile + gridDim.x, &s_desc[par ^ 1], &d);
+        if (f == 1) fill_rows<R, T>(s_desc[par ^ 1], rows + (par ^ 1) * G::NROW, tid);
+      }
+      Derivs v;
+      if (has_d2(f)) {
+        field_derivs<R, T, true, KO, 1, false, true>(cur + dz, T1, place, d, tid, v);
+        if (inside) {
+          double* const o = out + (long long)d2slot(f, 0) * n;
+#pragma unroll
+          for (int p = 0; p < 6; ++p) o[p * n] = v.d2[p];
+        }
+      } else {
+        field_derivs<R, T, false, KO, 1, false, true>(cur + dz, T1, place, d, tid, v);
+      }
+      if (inside) {
+        double* const o = out + (long long)d1slot(f, 0) * n;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) o[a * n] = __dmul_rn(v.s1[a], d.f1[a]);
+        if (KO) out[(long long)(NDERIV + f) * n] = v.ko;
+      }
+      double* t = cur; cur = nxt; nxt = t;
     }
+    par ^= 1;
   }
 }
 
@@ -427,11 +384,10 @@ int device_sms(int* sms) {
   return 0;
 }
 
-template <int R>
+template <int R, bool KO>
 int launch_deriv(const bssn::Args& a, cudaStream_t stream, int grid) {
-  using Geo = bssn::DerivGeom<R>;
-  const size_t smem = (size_t)Geo::VOL * sizeof(double);
-  auto kern = bssn::deriv_kernel<R>;
+  constexpr size_t smem = bssn::DerivLayout<R>::SMEM;
+  auto kern = bssn::deriv_kernel<R, KO>;
   static int flags[kMaxDev] = {0};
   int rc = set_smem(kern, smem, flags);
   if (rc) return rc;
@@ -757,14 +713,14 @@ int bssn_b200_derivatives(void* stream, const double* F, const double* S, double
   if (use_ko && ko_order != 6 && ko_order != 8) return fail(BSSN_B200_EINVAL, "derivatives: ko_order must be 6 or 8");
   bssn::Args a{};
   int grid = 0;
-  int rc = prepare(&a, Sx, Sy, Sz, 4, &grid);
+  int rc = prepare(&a, Sx, Sy, Sz, 3, &grid);
   if (rc) return rc;
   a.F = F; a.S = S; a.OUT = DOUT;
   a.use_ko = use_ko ? 1 : 0;
   a.ko_sigma = use_ko ? ko_sigma : 0.0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (use_ko && ko_order == 8) return launch_deriv<4>(a, st, grid);
-  return launch_deriv<3>(a, st, grid);
+  if (use_ko && ko_order == 8) return launch_deriv<4, true>(a, st, grid);
+  return use_ko ? launch_deriv<3, true>(a, st, grid) : launch_deriv<3, false>(a, st, grid);
 }
 
 int bssn_b200_rhs_algebra(void* stream, const double* F, const double* D, const double* S, double* OUT,

@@ -482,7 +482,9 @@ __device__ __forceinline__ void column_sums(const double* __restrict__ p, int st
 
 // One field's first-derivative sums s1 (unscaled), scaled second derivatives
 // and KO term at this thread's point. WAIT: also wait for the point values.
-template <int R, class T, bool D2, bool KO, int BAR, bool WAIT>
+// ROUND: the KO axes are added with a rounding each (the derivative bundle's
+// stated arithmetic) instead of fused.
+template <int R, class T, bool D2, bool KO, int BAR, bool WAIT, bool ROUND = false>
 __device__ __forceinline__ void field_derivs(const double* __restrict__ cur, double* __restrict__ T1,
                                              const PointPlace& pp, const TileDesc& w,
                                              int rt, Derivs& d) {
@@ -512,7 +514,8 @@ __device__ __forceinline__ void field_derivs(const double* __restrict__ cur, dou
         } else {
           sk = ko6_sum(v0, s1, s2, s3);
         }
-        d.ko = a == 0 ? __dmul_rn(sk, w.fk[a]) : __fma_rn(sk, w.fk[a], d.ko);
+        if (ROUND) d.ko = __dadd_rn(d.ko, __dmul_rn(sk, w.fk[a]));
+        else d.ko = a == 0 ? __dmul_rn(sk, w.fk[a]) : __fma_rn(sk, w.fk[a], d.ko);
       }
     }
   }
