@@ -92,6 +92,10 @@ const char* bssn_b200_version(void);
  * always 0. */
 int bssn_b200_async_copy_errors(int* count);
 
+/* S (device, 16 doubles) <- the 16 host scalars, read before the call returns
+ * and carried by the launch: enqueue only, no copy that waits for the stream. */
+int bssn_b200_set_scalars(void* stream, double* S, const double* host_scalars);
+
 /* The BSSN right-hand side: OUT = RHS(F) on every point of the padded grid.
  * Drop-in for the reference's fused FFI handler FusedImpl
  * (3D/src/bssn3d/cuda/rhs_fused.cu:22-53, bound as `Fused` at :55-61):

@@ -14,7 +14,7 @@ from typing import Dict, Tuple
 import torch
 
 from . import _lib
-from .fused_rhs import _stream_handle, as_device_state, device_scalars, pack_S
+from .fused_rhs import _stream_handle, as_device_state, stream_scalars, pack_S
 from .grid import Grid
 from .state import BSSNState
 
@@ -31,7 +31,7 @@ class ConstraintSolver:
     def constraints_tensor(self, state) -> torch.Tensor:
         U = as_device_state(state.data if isinstance(state, BSSNState) else state)
         g = self.grid
-        S = device_scalars(pack_S(2.0, 0.0, 1.0, g.dx, 0.0, 1.0, 0.0, (1, 1, 1, 1), (1, 0),
+        S = stream_scalars(pack_S(2.0, 0.0, 1.0, g.dx, 0.0, 1.0, 0.0, (1, 1, 1, 1), (1, 0),
                                   g.dy, g.dz), U.device)
         out = torch.empty((4,) + tuple(U.shape[1:]), dtype=torch.float64, device=U.device)
         _, Sx, Sy, Sz = U.shape
@@ -50,7 +50,7 @@ class ConstraintSolver:
         fixed-order reduction of its per-CTA partial sums."""
         U = as_device_state(state.data if isinstance(state, BSSNState) else state)
         g = self.grid
-        S = device_scalars(pack_S(2.0, 0.0, 1.0, g.dx, 0.0, 1.0, 0.0, (1, 1, 1, 1), (1, 0),
+        S = stream_scalars(pack_S(2.0, 0.0, 1.0, g.dx, 0.0, 1.0, 0.0, (1, 1, 1, 1), (1, 0),
                                   g.dy, g.dz), U.device)
         lib = _lib.load()
         out = torch.empty(2, dtype=torch.float64, device=U.device)

@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from . import _lib, msrk
-from .fused_rhs import _stream_handle, as_device_state, device_scalars, scalars
+from .fused_rhs import _stream_handle, as_device_state, stream_scalars, scalars
 from .grid import Grid
 from .rhs import BSSNSolver
 from .state import BSSNState, PhysicsParams
@@ -64,7 +64,7 @@ class BSSNEvolution:
 
     def _S(self, t: float, dt: float, device) -> torch.Tensor:
         g = self.grid
-        return device_scalars(scalars(self.params, g.dx, g.dy, g.dz, dt, t), device)
+        return stream_scalars(scalars(self.params, g.dx, g.dy, g.dz, dt, t), device)
 
     def _stage(self, stage, U, Y, ACC, YNEXT, S):
         lib = _lib.load()

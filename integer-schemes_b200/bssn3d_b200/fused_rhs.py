@@ -67,6 +67,22 @@ def device_scalars(S, device) -> torch.Tensor:
     return S.to(device).contiguous()
 
 
+def stream_scalars(S: np.ndarray, device) -> torch.Tensor:
+    """:func:`device_scalars` of a host pack for use on the current stream only:
+    the values travel as launch parameters of a one-warp kernel there, while a
+    copy from pageable memory waits for everything the stream holds."""
+    device = torch.device(device)
+    if device.type != "cuda":
+        return device_scalars(S, device)
+    S = np.ascontiguousarray(S, dtype=np.float64)
+    if S.size != NSCAL:
+        raise ValueError(f"fused: S must have {NSCAL} scalars, got {S.size}")
+    out = torch.empty(S.shape, dtype=torch.float64, device=device)
+    with torch.cuda.device(out.device):
+        _lib.check(_lib.load().bssn_b200_set_scalars(_stream_handle(out.device), out.data_ptr(), S.ctypes.data))
+    return out
+
+
 def rhs_tensor(Fs: torch.Tensor, S_dev: torch.Tensor, out: torch.Tensor = None) -> torch.Tensor:
     """OUT (24, Sx, Sy, Sz) = RHS of the stacked state (one kernel launch)."""
     lib = _lib.load()
@@ -85,10 +101,10 @@ def cuda_fused_algebra(F, dx, dy, dz, eta, lmbda, lambda_f, cahd_c, dt, ssl_h, s
     ``{field_name: d/dt}``; KO dissipation is not part of this call (it is the
     RK-stage entry's job, evolve.py:86-91)."""
     Fs = as_device_state(F)
-    S = device_scalars(pack_S(eta, cahd_c, dt, dx, ssl_h, ssl_sigma, t, lmbda, lambda_f, dy, dz),
+    S = stream_scalars(pack_S(eta, cahd_c, dt, dx, ssl_h, ssl_sigma, t, lmbda, lambda_f, dy, dz),
                        Fs.device)
     OUT = rhs_tensor(Fs, S)
-    return {OUTPUT_FIELDS[k]: OUT[k] for k in range(NOUT)}
+    return dict(zip(OUTPUT_FIELDS, OUT.unbind(0)))
 
 
 def device_rhs_fused(state, params, dx, dy, dz, dt, t=0.0):

@@ -187,6 +187,13 @@ __global__ void advance_time_kernel(double* S) {
   if (threadIdx.x == 0 && blockIdx.x == 0) S[6] = S[6] + S[2];
 }
 
+struct Scalars {
+  double v[16];
+};
+__global__ void set_scalars_kernel(double* __restrict__ S, const __grid_constant__ Scalars s) {
+  if (threadIdx.x < 16) S[threadIdx.x] = s.v[threadIdx.x];
+}
+
 // Algebra only: derivatives supplied by the caller (the reference's
 // algebra-only microbenchmark interface, 3D/src/bssn3d/cuda/gen_algebra_cuda.py:55-96),
 // consumed in the stream order of the fused kernel.
@@ -552,6 +559,16 @@ const char* bssn_b200_version(void) { return "bssn_b200 0.3 sm_100a"; }
 int bssn_b200_async_copy_errors(int* count) {
   if (!count) return fail(BSSN_B200_EINVAL, "async_copy_errors: NULL operand");
   *count = 0;
+  return 0;
+}
+
+int bssn_b200_set_scalars(void* stream, double* S, const double* host_scalars) {
+  if (!S || !host_scalars) return fail(BSSN_B200_EINVAL, "set_scalars: NULL operand");
+  bssn::Scalars s;
+  std::memcpy(s.v, host_scalars, sizeof(s.v));
+  bssn::set_scalars_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(S, s);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("set_scalars launch", e);
   return 0;
 }
 

@@ -77,3 +77,18 @@ def test_block_tiles_cover_the_core(variant, core, n):
     written = np.isfinite(got[0])
     assert written.sum() == n ** 3 and written[inner[1:]].all()   # the core and nothing else
     assert O.normwise_rel(got[inner], O.rhs(F, S)[inner]).max() < 1e-12
+
+
+def test_host_scalars_reach_the_device_in_stream_order():
+    from bssn3d_b200.fused_rhs import stream_scalars
+    want = np.random.default_rng(3).standard_normal(16)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        got = stream_scalars(want, "cuda")
+        want_then = want.copy()
+        want[:] = 0.0            # read before the call returned
+        copy = got.clone()       # ordered after it on the same stream
+    side.synchronize()
+    assert np.array_equal(copy.cpu().numpy(), want_then)
+    with pytest.raises(ValueError):
+        stream_scalars(np.zeros(15), "cuda")
