@@ -493,9 +493,7 @@ class BatchedEvolution:
 def autotune(evo: BatchedEvolution, U, dt: float, variants=None, orders=None, reps: int = 3):
     """Time one captured RK4 step for every (tile variant, block order) on
     this block list and keep the fastest. The tile shape and the block-to-CTA
-    mapping are the kernel's launch knobs; its register cap is fixed at one
-    255-register CTA per SM (a two-CTA, 128-register build of the same kernel
-    spills ~3.7 KB per thread and measured slower on B200). Returns
+    mapping are the kernel's launch knobs. Returns
     {(variant, order): ms} and leaves ``evo`` on the winner."""
     import torch
     from . import _lib

@@ -20,8 +20,8 @@
 // through shared memory and goes on with the next tile while the transport
 // role closes this one.
 //
-// What bounds it: latency at 16 warps, then the shared-memory pipe (65 % of
-// its wavefronts at 96^3 + ghosts; 24 % of the FP64 pipe, 1.35 instructions a
+// What bounds it: latency at 16 warps, then the shared-memory pipe (59 % of
+// its wavefronts on a 102^3 array; 24 % of the FP64 pipe, 1.34 instructions a
 // cycle). A 134^3 array, RK4 stage 1 with KO6: 2.30 ms for the one-thread-per-
 // point form with 8 warps (255 registers), 1.69 ms now; RHS 2.00 -> 1.34 ms;
 // constraints 1.69 -> 0.88 ms; KO order 8 3.42 -> 1.92 ms. Measured and not
