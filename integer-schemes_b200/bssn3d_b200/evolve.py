@@ -66,16 +66,25 @@ class BSSNEvolution:
         g = self.grid
         return stream_scalars(scalars(self.params, g.dx, g.dy, g.dz, dt, t), device)
 
+    def _synced(self, U, Y):
+        """Y with its periodic ghosts. A stage buffer is synced in place (its
+        ghosts are read by this stage only); the state itself goes through a
+        copy, its ghost values enter the update unsynced."""
+        b = self._buffers(U)
+        src = Y
+        if not any(Y is b[k] for k in ("Ya", "Yb")):
+            src = b["Ys"]
+            src.copy_(Y)
+        _, Sx, Sy, Sz = U.shape
+        _lib.check(_lib.load().bssn_b200_periodic_sync(_stream_handle(U.device), src.data_ptr(), Sx, Sy, Sz, self.ng))
+        return src
+
     def _stage(self, stage, U, Y, ACC, YNEXT, S):
         lib = _lib.load()
         _, Sx, Sy, Sz = U.shape
         src = Y
         if self.bc == "periodic":
-            Ys = self._buffers(U)["Ys"]
-            Ys.copy_(Y)
-            _lib.check(lib.bssn_b200_periodic_sync(_stream_handle(U.device), Ys.data_ptr(),
-                                                   Sx, Sy, Sz, self.ng))
-            src = Ys
+            src = self._synced(U, Y)
         p = self.params
         rc = lib.bssn_b200_rk4_stage(_stream_handle(U.device), stage, U.data_ptr(), src.data_ptr(),
                                      ACC.data_ptr(), YNEXT.data_ptr(), S.data_ptr(),
@@ -88,11 +97,7 @@ class BSSNEvolution:
         _, Sx, Sy, Sz = U.shape
         src = Y
         if self.bc == "periodic":
-            Ys = self._buffers(U)["Ys"]
-            Ys.copy_(Y)
-            _lib.check(lib.bssn_b200_periodic_sync(_stream_handle(U.device), Ys.data_ptr(),
-                                                   Sx, Sy, Sz, self.ng))
-            src = Ys
+            src = self._synced(U, Y)
         p = self.params
         ptr = lambda t: None if t is None else t.data_ptr()
         rc = lib.bssn_b200_msrk_stage(_stream_handle(U.device), stage, U.data_ptr(), src.data_ptr(),

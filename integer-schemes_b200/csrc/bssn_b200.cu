@@ -332,24 +332,26 @@ __global__ void enforce_kernel(double* __restrict__ U, long long n, double chi_f
   }
 }
 
-// One axis of the periodic ghost sync: ghosts [0,ng) <- [S-2ng, S-ng), [S-ng,S) <- [ng, 2ng).
-__global__ void periodic_axis_kernel(double* __restrict__ U, long long Sx, long long Sy, long long Sz, int axis, int ng) {
-  const long long S[3] = {Sx, Sy, Sz};
-  const long long st[3] = {Sy * Sz, Sz, 1};
-  const long long n = Sx * Sy * Sz;
-  const long long o1 = S[(axis + 1) % 3], o2 = S[(axis + 2) % 3];
-  const long long per_field = 2LL * ng * o1 * o2;
-  const long long total = per_field * NFIELD;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
-    const int f = (int)(q / per_field);
-    long long r = q % per_field;
-    const long long i2 = r % o2; r /= o2;
-    const long long i1 = r % o1; r /= o1;
-    const int layer = (int)r;  // 0..2ng-1
-    const long long cdst = layer < ng ? layer : S[axis] - 2 * ng + layer;
-    const long long csrc = layer < ng ? S[axis] - 2 * ng + layer : layer;
-    const long long base = i1 * st[(axis + 1) % 3] + i2 * st[(axis + 2) % 3];
-    U[f * n + base + cdst * st[axis]] = U[f * n + base + csrc * st[axis]];
+// Periodic ghost sync in one pass. The axis-by-axis sync (ghosts [0, ng) <-
+// [S - 2 ng, S - ng), [S - ng, S) <- [ng, 2 ng), x then y then z) leaves every
+// ghost point with the interior value at its index wrapped on all three axes,
+// so each point takes it directly: one launch that reads interiors and writes
+// ghosts, instead of three that each wait for the last. A thread takes one
+// point and moves its 24 fields. With the stage buffers synced in place, a
+// 49x56x64 RK4 step: 872 -> 733 us.
+__global__ void periodic_kernel(double* __restrict__ U, int Sx, int Sy, int Sz, int ng) {
+  const long long n = (long long)Sx * Sy * Sz;
+  auto wrap = [&](int c, int S) { return c < ng ? c + S - 2 * ng : (c >= S - ng ? c - (S - 2 * ng) : c); };
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    const int p = (int)q, z = p % Sz, t = p / Sz, y = t % Sy, x = t / Sy;  // fewer than 2^31 points (check_grid)
+    const int wx = wrap(x, Sx), wy = wrap(y, Sy), wz = wrap(z, Sz);
+    if (wx == x && wy == y && wz == z) continue;
+    const long long src = ((long long)wx * Sy + wy) * Sz + wz;
+    double v[NFIELD];
+#pragma unroll
+    for (int f = 0; f < NFIELD; ++f) v[f] = U[f * n + src];
+#pragma unroll
+    for (int f = 0; f < NFIELD; ++f) U[f * n + q] = v[f];
   }
 }
 
@@ -815,11 +817,10 @@ int bssn_b200_periodic_sync(void* stream, double* U, long long Sx, long long Sy,
   rc = device_sms(&sms);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  for (int axis = 0; axis < 3; ++axis) {
-    bssn::periodic_axis_kernel<<<sms * 4, 256, 0, st>>>(U, Sx, Sy, Sz, axis, ng);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail("periodic_sync launch", e);
-  }
+  const long long blocks = (Sx * Sy * Sz + 255) / 256, cap = 8LL * sms;
+  bssn::periodic_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(U, (int)Sx, (int)Sy, (int)Sz, ng);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail("periodic_sync launch", e);
   return 0;
 }
 

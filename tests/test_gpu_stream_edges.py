@@ -92,3 +92,12 @@ def test_host_scalars_reach_the_device_in_stream_order():
     assert np.array_equal(copy.cpu().numpy(), want_then)
     with pytest.raises(ValueError):
         stream_scalars(np.zeros(15), "cuda")
+
+
+@pytest.mark.parametrize("shape,ng", [((9, 9, 9), 3), ((12, 13, 17), 4), ((3, 4, 5), 1), ((40, 11, 66), 3)])
+def test_periodic_sync_in_one_pass(shape, ng):
+    from bssn3d_b200 import _lib
+    F = np.random.default_rng(ng).standard_normal((24,) + shape)
+    Fd = torch.from_numpy(F).cuda()
+    _lib.check(_lib.load().bssn_b200_periodic_sync(torch.cuda.current_stream().cuda_stream, Fd.data_ptr(), *shape, ng))
+    np.testing.assert_array_equal(Fd.cpu().numpy(), O.periodic_sync(F, ng))
