@@ -43,7 +43,9 @@ typedef struct bssn_b200_block {
   double h[3];      /* grid spacing dx, dy, dz */
   int core;         /* ghost layers the batched kernels leave alone: tiles cover
                        [core, s - core) on each axis (0 = the whole array; set it
-                       to the ghost width when bssn_b200_fill supplies the ghosts) */
+                       to the ghost width when bssn_b200_fill supplies the ghosts).
+                       A margin narrower than the stencil's reach (3; 4 with KO
+                       order 8) is allowed: indices are clamped at the array ends */
   int reserved;     /* 0 */
 } bssn_b200_block;
 

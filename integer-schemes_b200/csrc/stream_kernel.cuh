@@ -648,8 +648,10 @@ __global__ void __launch_bounds__(2 * NTHREADS, 1) stream_kernel(const __grid_co
     Fz = args.F + (d.base + z);
     nfield = (unsigned)d.n;
     whole = d.al && z >= 0 && z + 1 < d.sz;
-    // pairs past the array that no covered point reads stay as they are
-    copies = splace.row0 < G::NROW && z < d.sz + (d.core ? 0 : R);
+    // The last covered point, sz - 1 - core, reads R further: pairs past that
+    // stay as they are (inside the array they are copied all the same, so that
+    // a margin of R or more needs no cells past its end).
+    copies = splace.row0 < G::NROW && z < d.sz + max(R - d.core, 0);
   };
   using AllRows = std::true_type;
   using CrossRows = std::false_type;

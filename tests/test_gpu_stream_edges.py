@@ -52,22 +52,29 @@ def test_stage_rate_at_tile_edges(shape, ko):
     assert np.abs(nxt.cpu().numpy() - (F + 0.5 * S[2] * got)).max() <= 4 * np.finfo(float).eps * np.abs(F).max()
 
 
-@pytest.mark.parametrize("variant", [0, 1, 2, 3])
-@pytest.mark.parametrize("core,n", [(0, 13), (3, 10), (3, 17), (4, 12), (5, 11)])
-def test_block_tiles_cover_the_core(variant, core, n):
+def _one_block(shape, core, variant):
+    """A block table of one block (device tensor) and its tile count."""
     import ctypes
     from bssn3d_b200 import _lib
     from bssn3d_b200.amr import BlockDesc
+    tab = (BlockDesc * 1)()
+    tab[0].sx, tab[0].sy, tab[0].sz = shape
+    tab[0].h[:] = H
+    tab[0].core = core
+    nt = _lib.load().bssn_b200_batch_plan(ctypes.addressof(tab), 1, variant)
+    return torch.frombuffer(bytearray(bytes(memoryview(tab).cast("B"))), dtype=torch.uint8).cuda(), nt
+
+
+# margins below, at and above the stencil's reach; even and odd z extents
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("core,n", [(0, 13), (1, 18), (1, 13), (2, 16), (2, 17), (3, 10), (3, 17), (4, 12), (5, 11)])
+def test_block_tiles_cover_the_core(variant, core, n):
+    from bssn3d_b200 import _lib
     lib = _lib.load()
     s = n + 2 * core
     F, S = _state((s, s, s), 7 * n + core), _S()
-    S[3] = S[13] = S[14] = S[15] = 0.1
-    tab = (BlockDesc * 1)()
-    tab[0].sx = tab[0].sy = tab[0].sz = s
-    tab[0].h[:] = [0.1] * 3
-    tab[0].core = core
-    nt = lib.bssn_b200_batch_plan(ctypes.addressof(tab), 1, variant)
-    dev = torch.frombuffer(bytearray(bytes(memoryview(tab).cast("B"))), dtype=torch.uint8).cuda()
+    S[3] = H[0]                      # a block's dx is its x spacing
+    dev, nt = _one_block((s, s, s), core, variant)
     Fd, Sd = torch.from_numpy(F).cuda(), torch.from_numpy(S).cuda()
     out = torch.full_like(Fd, np.nan)
     _lib.check(lib.bssn_b200_batch_rhs(torch.cuda.current_stream().cuda_stream, Fd.data_ptr(), Sd.data_ptr(),
@@ -77,6 +84,27 @@ def test_block_tiles_cover_the_core(variant, core, n):
     written = np.isfinite(got[0])
     assert written.sum() == n ** 3 and written[inner[1:]].all()   # the core and nothing else
     assert O.normwise_rel(got[inner], O.rhs(F, S)[inner]).max() < 1e-12
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("ko,core,n", [(ko, core, n) for ko in (6, 8) for core in (1, 2, 3, 4) for n in (14, 13)]
+                         + [(0, 2, 14), (0, 3, 13), (0, 0, 12), (6, 0, 12), (8, 0, 12), (8, 0, 13)])
+def test_block_stage_rate_for_every_margin(variant, ko, core, n):
+    from bssn3d_b200 import _lib
+    lib = _lib.load()
+    shape = (n + 2 * core,) * 3
+    F, S = _state(shape, 11 * n + core), _S()
+    sigma = 0.1 if ko else 0.0
+    want = O.rhs(F, S) + (O.ko(F, *H, sigma, ko) if ko else 0.0)
+    dev, nt = _one_block(shape, core, variant)
+    Fd, Sd = torch.from_numpy(F).cuda(), torch.from_numpy(S).cuda()
+    acc, nxt = torch.full_like(Fd, np.nan), torch.full_like(Fd, np.nan)
+    _lib.check(lib.bssn_b200_batch_rk4_stage(torch.cuda.current_stream().cuda_stream, 0, Fd.data_ptr(), Fd.data_ptr(),
+                                             acc.data_ptr(), nxt.data_ptr(), Sd.data_ptr(), sigma, ko or 6, 1e-4, 1e-4,
+                                             dev.data_ptr(), 1, nt, variant))
+    got, inner = acc.cpu().numpy(), (slice(None),) + (slice(core, core + n),) * 3
+    assert np.isfinite(got).sum() == 24 * n ** 3
+    assert O.normwise_rel(got[inner], want[inner]).max() < 1e-12
 
 
 def test_host_scalars_reach_the_device_in_stream_order():
