@@ -104,7 +104,10 @@ def cuda_fused_algebra(F, dx, dy, dz, eta, lmbda, lambda_f, cahd_c, dt, ssl_h, s
     S = stream_scalars(pack_S(eta, cahd_c, dt, dx, ssl_h, ssl_sigma, t, lmbda, lambda_f, dy, dz),
                        Fs.device)
     OUT = rhs_tensor(Fs, S)
-    return dict(zip(OUTPUT_FIELDS, OUT.unbind(0)))
+    # The fields in one operation. unsafe_split and not unbind: torch refuses an
+    # in-place operation on one of unbind's views with an operand that requires
+    # a gradient; its condition holds, as only the parts are handed out.
+    return dict(zip(OUTPUT_FIELDS, OUT.flatten(0, 1).unsafe_split(OUT.shape[1])))
 
 
 def device_rhs_fused(state, params, dx, dy, dz, dt, t=0.0):

@@ -129,3 +129,17 @@ def test_periodic_sync_in_one_pass(shape, ng):
     Fd = torch.from_numpy(F).cuda()
     _lib.check(_lib.load().bssn_b200_periodic_sync(torch.cuda.current_stream().cuda_stream, Fd.data_ptr(), *shape, ng))
     np.testing.assert_array_equal(Fd.cpu().numpy(), O.periodic_sync(F, ng))
+
+
+def test_rates_take_in_place_operations_with_a_gradient():
+    from bssn3d_b200.fused_rhs import cuda_fused_algebra
+    from bssn3d_b200.state import FIELD_INPUTS
+    shape = (7, 8, 10)
+    F = torch.from_numpy(_state(shape, 3)).cuda()
+    rates = cuda_fused_algebra({n: F[k] for k, n in enumerate(FIELD_INPUTS)}, *H, 2.0, (1, 1, 1, 1), (1, 0),
+                               0.06, 0.02, 0.6, 20.0, 0.7)
+    rate = rates["chi"].clone()
+    w = torch.full(shape, 2.0, dtype=torch.float64, device="cuda", requires_grad=True)
+    rates["chi"].mul_(w)
+    rates["chi"].sum().backward()
+    assert torch.equal(w.grad, rate)
