@@ -158,7 +158,10 @@ class SlabEvolution:
         return U_local[:, self.layout.owned_slice()]
 
     def scalars(self, t: float, dt: float, device) -> torch.Tensor:
-        return self.evo._S(t, dt, device)
+        """The 16 scalars on ``device``, there when the call returns (usable on any stream)."""
+        from .fused_rhs import device_scalars, scalars
+        g = self.grid
+        return device_scalars(scalars(self.evo.params, g.dx, g.dy, g.dz, dt, t), device)
 
     def buffers(self, U: torch.Tensor):
         key = (tuple(U.shape), U.device)

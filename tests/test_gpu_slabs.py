@@ -41,3 +41,20 @@ def test_slabs_step_like_one_block(n, world, ko_order, ng):
     sums = sum(s.constraint_sums(G).cpu() for s, G in zip(slabs, got))
     h, m = torch.sqrt(sums[:2] / sums[2]).tolist()
     assert abs(h - h_ref) <= 1e-12 * h_ref and abs(m - m_ref) <= 1e-12 * m_ref
+
+
+def test_slab_scalars_are_there_when_the_call_returns():
+    from bssn3d_b200.grid import Grid
+    from bssn3d_b200.slabs import SlabEvolution
+    evo = SlabEvolution(Grid(Nx=8, Ny=8, Nz=8, dx=0.1, dy=0.1, dz=0.1, ng=3))
+    want = evo.scalars(0.25, 0.01, "cpu")
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        stale = [torch.full((16,), float("nan"), dtype=torch.float64, device="cuda") for _ in range(4)]
+        del stale
+        torch.cuda._sleep(200_000_000)       # about 0.1 s of work queued before the call
+        S = evo.scalars(0.25, 0.01, "cuda")
+    with torch.cuda.stream(other):
+        got = S.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(got.cpu(), want)
