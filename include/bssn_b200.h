@@ -95,7 +95,9 @@ const char* bssn_b200_version(void);
 int bssn_b200_async_copy_errors(int* count);
 
 /* S (device, 16 doubles) <- the 16 host scalars, read before the call returns
- * and carried by the launch: enqueue only, no copy that waits for the stream. */
+ * and carried by the launch: enqueue only, no copy that waits for the stream.
+ * A launch captured into a graph replays the values it was captured with (the
+ * Python calls that use it refuse to be captured for that reason). */
 int bssn_b200_set_scalars(void* stream, double* S, const double* host_scalars);
 
 /* The BSSN right-hand side: OUT = RHS(F) on every point of the padded grid.

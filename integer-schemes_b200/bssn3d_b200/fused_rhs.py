@@ -70,15 +70,20 @@ def device_scalars(S, device) -> torch.Tensor:
 def stream_scalars(S: np.ndarray, device) -> torch.Tensor:
     """:func:`device_scalars` of a host pack for use on the current stream only:
     the values travel as launch parameters of a one-warp kernel there, while a
-    copy from pageable memory waits for everything the stream holds."""
+    copy from pageable memory waits for everything the stream holds. Like that
+    copy it is refused under stream capture: every replay would repeat the
+    scalars of the capture, its time t among them."""
     device = torch.device(device)
     if device.type != "cuda":
         return device_scalars(S, device)
     S = np.ascontiguousarray(S, dtype=np.float64)
     if S.size != NSCAL:
         raise ValueError(f"fused: S must have {NSCAL} scalars, got {S.size}")
-    out = torch.empty(S.shape, dtype=torch.float64, device=device)
-    with torch.cuda.device(out.device):
+    with torch.cuda.device(device):
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("fused: host scalars cannot enter a captured graph, it would replay their values; "
+                               "capture calls that take device scalars (BSSNEvolution.capture, rhs_tensor)")
+        out = torch.empty(S.shape, dtype=torch.float64, device=device)
         _lib.check(_lib.load().bssn_b200_set_scalars(_stream_handle(out.device), out.data_ptr(), S.ctypes.data))
     return out
 

@@ -143,3 +143,25 @@ def test_rates_take_in_place_operations_with_a_gradient():
     rates["chi"].mul_(w)
     rates["chi"].sum().backward()
     assert torch.equal(w.grad, rate)
+
+
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+@pytest.mark.parametrize("call", ["rhs_dict", "step", "constraints"])
+def test_scalars_are_refused_under_capture(call):
+    from bssn3d_b200.constraints import ConstraintSolver
+    from bssn3d_b200.evolve import BSSNEvolution
+    from bssn3d_b200.grid import Grid
+    from bssn3d_b200.rhs import BSSNSolver
+    from bssn3d_b200.state import BSSNState
+    grid = Grid(Nx=8, Ny=8, Nz=8, dx=0.1, dy=0.1, dz=0.1, ng=3)
+    state = BSSNState(torch.from_numpy(_state((14, 14, 14), 2)).cuda())
+    fn = {"rhs_dict": lambda: BSSNSolver(grid, dt=0.02, ko_order=6).rhs_dict(state, 0.3, 0.02),
+          "step": lambda: BSSNEvolution(grid, ko_sigma=0.1, ko_order=6, bc="none").step(state, 0.3, 0.02).data,
+          "constraints": lambda: ConstraintSolver(grid).constraints_tensor(state)}[call]
+    fn()
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="captur"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            fn()
+    torch.cuda.synchronize()
+    fn()
