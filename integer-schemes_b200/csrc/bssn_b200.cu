@@ -41,29 +41,17 @@ __device__ __forceinline__ bool hold_for_enforce(double* en, int k, double un) {
   return true;
 }
 
-// Algebraic enforcement of one point (evolve.py:93-119): unit conformal
-// determinant, traceless A~ with the unit-det inverse, chi and alpha floors.
-__device__ __forceinline__ void enforce_point(double* en, double* O, long long n, double chi_floor,
-                                              double alpha_floor) {
-  double* g = en;
-  double* a = en + 6;
-  const double det = g[0] * (g[3] * g[5] - g[4] * g[4]) - g[1] * (g[1] * g[5] - g[4] * g[2]) +
-                     g[2] * (g[1] * g[4] - g[3] * g[2]);
-  const double scale = pow(det, -1.0 / 3.0);
+// Enforces the held values of one point and stores them.
+__device__ __forceinline__ void store_enforced(double (&en)[14], double* O, long long n, double chi_floor,
+                                               double alpha_floor) {
+  double v[12];
 #pragma unroll
-  for (int q = 0; q < 6; ++q) g[q] = g[q] * scale;
-  const double iuxx = g[3] * g[5] - g[4] * g[4];
-  const double iuxy = g[2] * g[4] - g[1] * g[5];
-  const double iuxz = g[1] * g[4] - g[2] * g[3];
-  const double iuyy = g[0] * g[5] - g[2] * g[2];
-  const double iuyz = g[1] * g[2] - g[0] * g[4];
-  const double iuzz = g[0] * g[3] - g[1] * g[1];
-  const double trA = iuxx * a[0] + iuyy * a[3] + iuzz * a[5] + 2.0 * (iuxy * a[1] + iuxz * a[2] + iuyz * a[4]);
-  const double third = trA / 3.0;
+  for (int q = 0; q < 12; ++q) v[q] = en[q];
+  enforce_metric(v);
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
-    O[(long long)(F_GT + q) * n] = g[q];
-    O[(long long)(F_AT + q) * n] = a[q] - g[q] * third;
+    O[(long long)(F_GT + q) * n] = v[q];
+    O[(long long)(F_AT + q) * n] = v[6 + q];
   }
   O[(long long)F_CHI * n] = fmax(en[12], chi_floor);
   O[(long long)F_ALPHA * n] = fmax(en[13], alpha_floor);
@@ -300,33 +288,18 @@ __global__ void __launch_bounds__(128) stage_derivs_kernel(
       }
     };
     acc.finalize(fld, P, emit);
-    if (stage == 3) enforce_point(en, O, n, chi_floor, alpha_floor);
+    if (stage == 3) store_enforced(en, O, n, chi_floor, alpha_floor);
   }
 }
 
 __global__ void enforce_kernel(double* __restrict__ U, long long n, double chi_floor, double alpha_floor) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    double g[6], a[6];
+    double v[12];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) { g[k] = U[(F_GT + k) * n + q]; a[k] = U[(F_AT + k) * n + q]; }
-    const double det = g[0] * (g[3] * g[5] - g[4] * g[4]) - g[1] * (g[1] * g[5] - g[4] * g[2]) +
-                       g[2] * (g[1] * g[4] - g[3] * g[2]);
-    const double scale = pow(det, -1.0 / 3.0);
+    for (int k = 0; k < 6; ++k) { v[k] = U[(F_GT + k) * n + q]; v[6 + k] = U[(F_AT + k) * n + q]; }
+    enforce_metric(v);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) g[k] = g[k] * scale;
-    const double iuxx = g[3] * g[5] - g[4] * g[4];
-    const double iuxy = g[2] * g[4] - g[1] * g[5];
-    const double iuxz = g[1] * g[4] - g[2] * g[3];
-    const double iuyy = g[0] * g[5] - g[2] * g[2];
-    const double iuyz = g[1] * g[2] - g[0] * g[4];
-    const double iuzz = g[0] * g[3] - g[1] * g[1];
-    const double trA = iuxx * a[0] + iuyy * a[3] + iuzz * a[5] + 2.0 * (iuxy * a[1] + iuxz * a[2] + iuyz * a[4]);
-    const double third = trA / 3.0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      U[(F_GT + k) * n + q] = g[k];
-      U[(F_AT + k) * n + q] = a[k] - g[k] * third;
-    }
+    for (int k = 0; k < 6; ++k) { U[(F_GT + k) * n + q] = v[k]; U[(F_AT + k) * n + q] = v[6 + k]; }
     U[F_CHI * n + q] = fmax(U[F_CHI * n + q], chi_floor);
     U[F_ALPHA * n + q] = fmax(U[F_ALPHA * n + q], alpha_floor);
   }

@@ -165,3 +165,42 @@ def test_scalars_are_refused_under_capture(call):
             fn()
     torch.cuda.synchronize()
     fn()
+
+
+def test_every_enforcement_gives_the_same_bytes():
+    from bssn3d_b200 import _lib
+    lib = _lib.load()
+    shape = (9, 10, 18)
+    F, S = _state(shape, 4), _S(dt=1e-300)   # the update itself leaves u as it is
+    S[1] = 0.0                                # no CAHD term: it divides by dt
+    U, Sd = torch.from_numpy(F).cuda(), torch.from_numpy(S).cuda()
+    st = torch.cuda.current_stream().cuda_stream
+    n = F[0].size
+    want = U.clone()
+    _lib.check(lib.bssn_b200_enforce(st, want.data_ptr(), n, 1e-4, 1e-4))
+    acc = torch.zeros_like(U)
+    fused = torch.empty_like(U)
+    _lib.check(lib.bssn_b200_rk4_stage(st, 3, U.data_ptr(), U.data_ptr(), acc.data_ptr(), fused.data_ptr(),
+                                       Sd.data_ptr(), 0.0, 6, 1e-4, 1e-4, *shape))
+    assert torch.equal(fused, want)
+    dev, _ = _one_block(shape, 0, 0)
+    D = torch.zeros((138,) + shape, dtype=torch.float64, device="cuda")
+    pts = torch.tensor([0, n], dtype=torch.int64, device="cuda")
+    out = torch.empty_like(U)
+    _lib.check(lib.bssn_b200_batch_rk4_stage_derivs(st, 3, U.data_ptr(), U.data_ptr(), acc.data_ptr(), out.data_ptr(),
+                                                    D.data_ptr(), Sd.data_ptr(), 0, 1e-4, 1e-4, dev.data_ptr(), 1,
+                                                    pts.data_ptr(), n))
+    assert torch.equal(out, want)
+
+
+def test_enforcement_of_degenerate_metrics():
+    """Zero, negative and overflowing determinants come out as the oracle's pow gives them."""
+    from bssn3d_b200 import _lib
+    F = _state((1, 1, 6), 9)
+    F[3:9] = 0.0
+    F[3, 0, 0] = [1.0, -1.0, 1e200, -1e200, 0.0, np.nan]
+    F[6, 0, 0] = F[8, 0, 0] = [1.0, 1.0, 1e200, 1e200, 0.0, 1.0]
+    U = torch.from_numpy(F).cuda()
+    _lib.check(_lib.load().bssn_b200_enforce(torch.cuda.current_stream().cuda_stream, U.data_ptr(), 6, 1e-4, 1e-4))
+    # 4 ulp: three products and a sum of A~'s trace
+    np.testing.assert_allclose(U.cpu().numpy(), O.enforce(F), rtol=4 * np.finfo(float).eps, atol=1e-17)
