@@ -91,7 +91,9 @@ const char* bssn_b200_version(void);
 
 /* Number of bulk-copy waits that gave up since the library was loaded. The
  * kernels stage their tiles with per-thread copies, which need no such wait:
- * always 0. */
+ * always 0, kept for callers of earlier versions. The environment variable
+ * BSSN_B200_STAGING, which chose bulk copies there (same results, slower), has
+ * no effect. */
 int bssn_b200_async_copy_errors(int* count);
 
 /* S (device, 16 doubles) <- the 16 host scalars, read before the call returns

@@ -9,6 +9,8 @@ The library is mandatory: there is no CPU or PyTorch fallback. If
 from __future__ import annotations
 
 import ctypes
+import os
+import warnings
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libbssn_b200.so"
@@ -75,6 +77,9 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = args
         fn.restype = res
+    if os.environ.get("BSSN_B200_STAGING") == "tma":
+        warnings.warn("BSSN_B200_STAGING=tma has no effect: the bulk-tensor staging it chose (same results, slower) "
+                      "is no longer built", RuntimeWarning, stacklevel=2)
     _lib = lib
     return lib
 

@@ -56,6 +56,13 @@ def test_missing_library_raises(monkeypatch, tmp_path):
         _lib.load()
 
 
+def test_a_staging_choice_without_effect_is_reported(monkeypatch):
+    monkeypatch.setenv("BSSN_B200_STAGING", "tma")
+    monkeypatch.setattr(_lib, "_lib", None)
+    with pytest.warns(RuntimeWarning, match="no effect"):
+        _lib.load()
+
+
 def test_solver_validation():
     from bssn3d_b200.rhs import BSSNSolver
     g3 = Grid.from_domain(16, ng=3)
