@@ -312,6 +312,12 @@ def bench_reference(args):
     world, rank, _ = dist_env()
     if rank != 0:
         return
+    from oracle import oracle as O
+    if not O.have_ref():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": f"{O.REF_PATH.relative_to(ROOT)} not built: `make -C oracle ref` needs the "
+                                         "reference's sources"}), flush=True)
+        return
     threads = cpu_threads()
     U, S, interior = reference_step_sample(args.n)
     times = run_cpu_reference(U, S, args.steps, args.warmup, threads)

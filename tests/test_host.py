@@ -108,3 +108,15 @@ def test_physics_defaults():
     p = PhysicsParams()
     assert (p.eta, p.lmbda, p.lambda_f, p.cahd_c, p.ssl_h, p.ssl_sigma) == \
         (2.0, (1.0, 1.0, 1.0, 1.0), (1.0, 0.0), 0.06, 0.6, 20.0)
+
+
+def test_reference_arm_says_when_the_reference_is_not_built(monkeypatch, capsys):
+    import argparse
+    import json
+    import bench
+    from oracle import oracle as O
+    monkeypatch.setattr(O, "REF_PATH", ROOT / "oracle" / "_ref" / "absent.so")
+    monkeypatch.setattr(O, "_ref", None)
+    bench.bench_reference(argparse.Namespace(n=16, steps=1, warmup=0, gpus=1))
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "absent.so" in line["unavailable"]
