@@ -1,14 +1,10 @@
-"""Halo staging of the stream kernel by bulk-tensor (TMA) copies
-(BSSN_B200_STAGING=tma).
+"""Staging of the stream kernel and the derivative bundle by aligned 16-byte
+pairs against clamped 8-byte copies.
 
-With the knob set, a state whose z extent is even and whose base is 16-byte
-aligned is staged by one bulk-tensor copy per field and tile (edge tiles are
-then clamped in shared memory); a state placed 8 bytes off a 16-byte boundary
-cannot be, so it takes the default per-thread cp.async staging. Both paths
-must give the same bytes for every kernel mode, and no bounded copy wait may
-give up."""
-
-import ctypes
+A state whose z extent is even and whose base is 16-byte aligned is staged in
+16-byte pairs wherever a pair lies inside the array; the same state placed 8
+bytes off a 16-byte boundary goes entirely in 8-byte copies. Both must give the
+same bytes for every kernel mode."""
 
 import numpy as np
 import pytest
@@ -19,11 +15,6 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 SHAPE = (18, 22, 64)   # interior and edge tiles on every axis
-
-
-@pytest.fixture(autouse=True)
-def _bulk_copy_staging(monkeypatch):
-    monkeypatch.setenv("BSSN_B200_STAGING", "tma")
 
 
 def _lib():
@@ -84,26 +75,24 @@ def _run(kind, aligned, ko_order=6, stage=1):
         L.check(lib.bssn_b200_constraint_norms(stream, Fd.data_ptr(), S.data_ptr(), Sx, Sy, Sz, 3,
                                                scratch.data_ptr(), need, out.data_ptr()))
         return out.cpu().numpy()
+    if kind == "derivs":
+        out = torch.empty((162,) + SHAPE, dtype=torch.float64, device="cuda")
+        L.check(lib.bssn_b200_derivatives(stream, Fd.data_ptr(), S.data_ptr(), out.data_ptr(), 0.1, ko_order, Sx, Sy, Sz))
+        return out.cpu().numpy()
     raise ValueError(kind)
 
 
 @pytest.mark.parametrize("kind,ko_order,stage", [("rhs", 6, 0), ("constraints", 6, 0), ("norms", 6, 0),
-                                                 ("stage", 6, 1), ("stage", 6, 3), ("stage", 8, 2)])
-def test_bulk_copies_and_per_thread_staging_agree_bitwise(kind, ko_order, stage):
+                                                 ("stage", 6, 1), ("stage", 6, 3), ("stage", 8, 2),
+                                                 ("derivs", 6, 0), ("derivs", 8, 0)])
+def test_paired_and_single_copies_agree_bitwise(kind, ko_order, stage):
     a = _run(kind, True, ko_order, stage)
     b = _run(kind, False, ko_order, stage)
     assert np.isfinite(a).all()
     np.testing.assert_array_equal(a, b)
 
 
-def test_rhs_with_bulk_copies_vs_oracle():
+def test_rhs_with_paired_copies_vs_oracle():
     F = _state()
     got = _run("rhs", True)
     assert O.normwise_rel(got, O.rhs(F, _S())).max() < 1e-12
-
-
-def test_no_bounded_copy_wait_gave_up():
-    L, lib = _lib()
-    count = ctypes.c_int(-1)
-    L.check(lib.bssn_b200_async_copy_errors(ctypes.addressof(count)))
-    assert count.value == 0
