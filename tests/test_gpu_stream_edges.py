@@ -1,8 +1,10 @@
 """The two-role stream kernel where it can go wrong: tiles that hang over every
 end of the array, extents below one tile, odd z extents (no aligned rows) and
 even ones (16-byte copies with clamped ends), more tiles than CTAs, every
-instantiation of the stage (no KO, KO 6, KO 8), all tile shapes on blocks with
-and without a ghost margin.
+instantiation of the stage (no KO, KO 6, KO 8), all tile shapes (and with them
+every shared-memory layout and its barriers) on blocks with and without a ghost
+margin, on single blocks and on lists whose CTAs go from block to block; NaN and
+infinity, which must stay within the stencil; the calls around the kernel.
 
 Bars as in test_gpu_parity.py: 1e-12 of each field's largest rate (a second
 derivative of O(1) data carries eps / h^2 = 2e-14, times at most ~50 terms)."""
@@ -30,7 +32,8 @@ def _state(shape, seed):
     return F
 
 
-SHAPES = [(1, 1, 1), (2, 3, 5), (4, 4, 16), (5, 3, 17), (3, 9, 18), (8, 4, 33), (23, 26, 34)]
+SHAPES = [(1, 1, 1), (2, 3, 5), (4, 4, 16), (5, 3, 17), (3, 9, 18), (8, 4, 33), (23, 26, 34),
+          (29, 30, 50), (30, 29, 51)]   # the last two: 256 tiles, more than CTAs
 
 
 @pytest.mark.parametrize("shape", SHAPES)
@@ -105,6 +108,95 @@ def test_block_stage_rate_for_every_margin(variant, ko, core, n):
     got, inner = acc.cpu().numpy(), (slice(None),) + (slice(core, core + n),) * 3
     assert np.isfinite(got).sum() == 24 * n ** 3
     assert O.normwise_rel(got[inner], want[inner]).max() < 1e-12
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+@pytest.mark.parametrize("ko", [0, 6, 8])
+@pytest.mark.parametrize("margin", [False, True])
+def test_block_list_stages_from_block_to_block(variant, ko, margin):
+    """Six blocks of unequal shape and spacing, some at odd offsets, in more tiles
+    than CTAs: first and last stage against the oracle."""
+    import ctypes
+    from bssn3d_b200 import _lib
+    from bssn3d_b200.amr import BlockDesc
+    lib = _lib.load()
+    core = 0 if not margin else (4 if ko == 8 else 3)
+    inner = [(24, 22, 26), (9, 11, 13), (30, 16, 24), (5, 6, 40), (17, 18, 19), (26, 25, 24)]
+    shapes = [tuple(n + 2 * core for n in c) for c in inner]
+    tab, at, size = (BlockDesc * len(shapes))(), [], 0
+    for b, shape in enumerate(shapes):
+        size += b % 2                     # odd offsets for every other pair of blocks
+        at.append(size)
+        tab[b].offset, tab[b].core = size, core
+        tab[b].sx, tab[b].sy, tab[b].sz = shape
+        tab[b].h[:] = [h * (1 + 0.25 * b) for h in H]
+        size += 24 * int(np.prod(shape))
+    nt = lib.bssn_b200_batch_plan(ctypes.addressof(tab), len(shapes), variant)
+    assert nt > torch.cuda.get_device_properties(0).multi_processor_count
+    dev = torch.frombuffer(bytearray(bytes(memoryview(tab).cast("B"))), dtype=torch.uint8).cuda()
+    view = lambda P, b: P[at[b]:at[b] + 24 * int(np.prod(shapes[b]))].reshape((24,) + shapes[b])  # noqa: E731
+    Y, U, A = np.zeros(size), np.zeros(size), np.zeros(size)
+    for b, shape in enumerate(shapes):
+        view(Y, b)[:], view(U, b)[:], view(A, b)[:] = (_state(shape, 31 * b + k) for k in range(3))
+    sigma, S = (0.1 if ko else 0.0), _S()
+    Sd, Yd, Ud = (torch.from_numpy(x).cuda() for x in (S, Y, U))
+    for stage in (0, 3):
+        Ad, Od = torch.from_numpy(A).cuda(), torch.full((size,), np.nan, dtype=torch.float64, device="cuda")
+        _lib.check(lib.bssn_b200_batch_rk4_stage(
+            torch.cuda.current_stream().cuda_stream, stage, Ud.data_ptr(), Yd.data_ptr(), Ad.data_ptr(), Od.data_ptr(),
+            Sd.data_ptr(), sigma, ko or 6, 1e-4, 1e-4, dev.data_ptr(), len(shapes), nt, variant))
+        acc, out = Ad.cpu().numpy(), Od.cpu().numpy()
+        for b, c in enumerate(inner):
+            h = [x * (1 + 0.25 * b) for x in H]
+            s = S.copy()
+            s[3], s[13:16], s[6] = h[0], h, S[6] + (S[2] if stage == 3 else 0.0)
+            rate = O.rhs(view(Y, b), s) + (O.ko(view(Y, b), *h, sigma, ko) if ko else 0.0)
+            I = (slice(None),) + tuple(slice(core, core + m) for m in c)
+            got = view(out, b)
+            assert np.isfinite(got).sum() == 24 * np.prod(c)          # the core and nothing else
+            if stage == 0:
+                assert O.normwise_rel(view(acc, b)[I], rate[I]).max() < 1e-12
+                want = view(U, b) + 0.5 * S[2] * rate
+            else:
+                want = O.enforce(view(U, b) + (S[2] / 6.0) * (view(A, b) + rate))
+            assert O.normwise_rel_grouped(got[I], want[I]).max() < 1e-12
+
+
+@pytest.mark.parametrize("ko", [0, 6, 8])
+@pytest.mark.parametrize("shape", [(41, 45, 84), (45, 41, 85)])
+def test_derivative_bundle_with_several_tiles_a_cta(shape, ko):
+    """792 tiles on 444 CTAs: the hand-over of descriptor and row table, bit for bit."""
+    from bssn3d_b200.fused_rhs import derivatives, device_scalars
+    F = _state(shape, 5)
+    D = derivatives(torch.from_numpy(F).cuda(), device_scalars(_S(), "cuda"), ko_sigma=0.1 if ko else 0.0,
+                    ko_order=ko or 6).cpu().numpy()
+    np.testing.assert_array_equal(D[:138], O.derivatives(F, *H))
+    if ko:
+        np.testing.assert_array_equal(D[138:], O.ko(F, *H, 0.1, ko))
+
+
+@pytest.mark.parametrize("ko", [6, 8])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("field", [1, 4, 2, 9, 13, 22])     # chi, gt, K, beta, At, B: both roles, with and without mixed taps
+@pytest.mark.parametrize("shape,at", [((13, 14, 20), (6, 6, 9)), ((13, 14, 21), (12, 13, 20)), ((9, 14, 20), (0, 0, 0)),
+                                      ((9, 14, 34), (3, 4, 33))])
+def test_nonfinite_values_stay_within_the_stencil(shape, at, field, bad, ko):
+    from bssn3d_b200 import _lib
+    lib = _lib.load()
+    F, Sd = _state(shape, 12), torch.from_numpy(_S()).cuda()
+    outs = []
+    for value in (F[(field,) + at], bad):
+        F[(field,) + at] = value
+        Fd = torch.from_numpy(F).cuda()
+        acc, nxt = torch.empty_like(Fd), torch.empty_like(Fd)
+        _lib.check(lib.bssn_b200_rk4_stage(torch.cuda.current_stream().cuda_stream, 0, Fd.data_ptr(), Fd.data_ptr(),
+                                           acc.data_ptr(), nxt.data_ptr(), Sd.data_ptr(), 0.1, ko, 1e-4, 1e-4, *shape))
+        outs.append(acc.cpu().numpy())
+    # a stencil reaches ko / 2 points along one axis and 3 along two (none of these clamps past the value)
+    dist = np.sort(np.abs(np.indices(shape) - np.reshape(at, (3, 1, 1, 1))), axis=0)
+    reach = (dist[0] == 0) & (((dist[1] == 0) & (dist[2] <= ko // 2)) | (dist[2] <= 3))
+    np.testing.assert_array_equal(outs[1][:, ~reach], outs[0][:, ~reach])
+    assert not np.isfinite(outs[1][(field,) + at])
 
 
 def test_host_scalars_reach_the_device_in_stream_order():
