@@ -60,7 +60,7 @@ struct Shape {
 };
 using DefaultShape = Shape<4, 4, 16>;
 
-enum Mode : int { MODE_DERIV = 0, MODE_RHS = 1, MODE_STAGE = 2, MODE_CON = 3, MODE_NORM = 4, MODE_MSRK = 5 };
+enum Mode : int { MODE_RHS = 1, MODE_STAGE = 2, MODE_CON = 3, MODE_NORM = 4, MODE_MSRK = 5 };
 
 struct Args {
   const double* F;  // stage input (24, n)
@@ -201,15 +201,20 @@ struct TileGeom {
     return (size_t)(nbuf * VOL + 2 * TVOL) * sizeof(double) + slots(X_N + nslot) + TABLES;
   }
   static constexpr size_t CAP = 232448 - 832;  // shared memory per CTA less the static part
-  // The richest layout that fits. NB: buffers of the transport role (two or
-  // three). PIPE: the geometry role has its own point values and runs up to a
-  // tile ahead, else the roles share them. LEAN leaves At out of the point
-  // values (read from global memory where it is used): of the geometry role's
-  // (LEAN_A) or of both.
-  static constexpr int FIT = need(5, 18 + 17) <= CAP ? 0 : need(5, 18 + 11) <= CAP ? 1 : need(4, 18 + 17) <= CAP ? 2
-                           : need(4, 18 + 11) <= CAP ? 3 : need(4, 12 + 11) <= CAP ? 4 : need(4, 18) <= CAP ? 5 : 6;
-  static constexpr int NB = FIT <= 1 ? 3 : 2;
-  static constexpr bool PIPE = FIT <= 4, LEAN = FIT == 4 || FIT == 6, LEAN_A = LEAN || FIT == 1 || FIT == 3;
+  // The richest layout that fits: NB buffers of the transport role, and the
+  // geometry role's own copy of the point values (PIPE, it runs up to a tile
+  // ahead) or one copy for both roles. LEAN leaves At out of the point values
+  // (read from global memory where it is used): of the geometry role's (LEAN_A)
+  // or of both. In the order of the ladder, doubles per point in brackets:
+  //   0  three buffers, LEAN_A (18 + 11)     KO <= 6: 4x4x16
+  //   1  two buffers (18 + 17)               KO <= 6: 2x8x16
+  //   2  two buffers, LEAN_A (18 + 11)       KO 8: 4x4x16, 2x8x16
+  //   3  two buffers, LEAN (12 + 11)         KO <= 6: 4x8x8, 8x4x8
+  //   4  two buffers, LEAN, one copy (12)    KO 8: 4x8x8, 8x4x8
+  static constexpr int FIT = need(5, 18 + 11) <= CAP ? 0 : need(4, 18 + 17) <= CAP ? 1 : need(4, 18 + 11) <= CAP ? 2
+                           : need(4, 12 + 11) <= CAP ? 3 : 4;
+  static constexpr int NB = FIT == 0 ? 3 : 2;
+  static constexpr bool PIPE = FIT <= 3, LEAN = FIT >= 3, LEAN_A = FIT != 1;
   static constexpr int NPB = LEAN ? 12 : 18, NPA = PIPE ? (LEAN_A ? 11 : 17) : 0;
   static constexpr size_t SMEM = need(2 + NB, NPB + NPA);
   static_assert(SMEM <= CAP, "tile does not fit shared memory");
@@ -219,7 +224,7 @@ struct TileDesc {
   long long base, n;      // first double of the block, points per field
   int sx, sy, sz, core;
   int x0, y0, z0, zs;     // first point of the tile, first staged z
-  int al, pad;            // 16-byte row copies allowed
+  int al;                 // 16-byte row copies allowed
   double f1[3], f2[3], fk[3], fm[3];  // stencil scale factors (scales())
   double cahd;            // C dx^2 / (dt (10 dx^2 + 1))
   int tile0, tile_end;    // tiles of its block
