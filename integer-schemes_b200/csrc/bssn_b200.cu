@@ -60,12 +60,12 @@ __device__ __forceinline__ void store_enforced(double (&en)[14], double* O, long
 // ---------------------------------------------------------------------------
 // Derivative bundle to global memory (the bssn_b200_derivatives entry): the
 // staging and the stencils of the stream kernel, one field at a time,
-// double-buffered, every result stored at once. 1.5 KB are written and 0.2 KB
-// read per point, so the stores should be all that counts: three CTAs per SM
-// (85 registers, 49 KB each) keep them going while others differentiate. An
-// 86^3 array with KO6: 0.64 ms with single buffering, one 8-byte copy a cell
-// and 36 taps per mixed derivative, 0.43 ms now (2.2 TB/s; copy
-// latency and the shared-memory pipe bound it).
+// double-buffered, every result stored at once. 1.3 KB are written and 0.2 KB
+// read per point (KO on), so the stores should be all that counts: three CTAs
+// per SM (77-78 registers, 49 KB each) keep them going while others
+// differentiate. An 86^3 array with KO6: 0.64 ms with single buffering, one
+// 8-byte copy a cell and 36 taps per mixed derivative, 0.43 ms now (2.2 TB/s,
+// 1.9 of it stores; copy latency and the shared-memory pipe bound it).
 // ---------------------------------------------------------------------------
 template <int R>
 struct DerivLayout {
